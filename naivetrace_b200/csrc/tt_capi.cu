@@ -1046,9 +1046,10 @@ tt_status tt_upload_scene(tt_ctx* c) {
   s.num_point_lights = (int)c->points.size();
   // Environmental lights.
   s.num_env = (int)c->envs.size();
+  std::vector<DevEnvLight> denv(c->envs.size());
   for (size_t i = 0; i < c->envs.size(); ++i) {
     const tt_env_light& e = c->envs[i].desc;
-    DevEnvLight& L = s.env[i];
+    DevEnvLight& L = denv[i];
     std::memset(&L, 0, sizeof(L));
     L.kind = e.kind;
     double dir[3] = {e.dir[0], e.dir[1], e.dir[2]};
@@ -1122,6 +1123,7 @@ tt_status tt_upload_scene(tt_ctx* c) {
       L.guide_cols = (const int*)upload(gcols.data(), gcols.size() * sizeof(int));
     }
   }
+  s.env = (const DevEnvLight*)upload(denv.data(), denv.size() * sizeof(DevEnvLight));
   mark("env maps");
   // Camera (camera.hxx:38-108, 159-175), computed in double.
   s.cam = make_dev_camera(c->camera);

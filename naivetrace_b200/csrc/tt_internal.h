@@ -123,7 +123,8 @@ struct DevScene {
   int num_point_lights;
   int num_env;
   int num_tris;
-  DevEnvLight env[MAX_ENV_LIGHTS];
+  const DevEnvLight* env;     // num_env lights, in global memory: a warp's lanes pick different
+                              // lights and read their spectra at different bins
   DevCamera cam;
   float type_probs[4];        // ENV, AREA, POINT, VOLUME
   float in_class_area;

@@ -2168,13 +2168,14 @@ __global__ void k_eval_phase(DevScene sc, int medium, float3 pos, float3 wi, int
 
 
 void upload_constant_tables() {
-  float m[3][NBINS], smits[7][NBINS];
-  for (int i = 0; i < 3; ++i)
-    for (int b = 0; b < NBINS; ++b) m[i][b] = (float)kSpectrumToRgb[i][b];
-  for (int i = 0; i < 7; ++i)
-    for (int b = 0; b < NBINS; ++b) smits[i][b] = (float)kSmitsBasis[i][b];
-  cudaMemcpyToSymbol(c_spec_to_rgb, m, sizeof(m));
-  cudaMemcpyToSymbol(c_smits, smits, sizeof(smits));
+  float4 m[NBINS];
+  float smits[NBINS][8];
+  for (int b = 0; b < NBINS; ++b) {
+    m[b] = make_float4((float)kSpectrumToRgb[0][b], (float)kSpectrumToRgb[1][b], (float)kSpectrumToRgb[2][b], 0.f);
+    for (int i = 0; i < 8; ++i) smits[b][i] = i < 7 ? (float)kSmitsBasis[i][b] : 0.f;
+  }
+  cudaMemcpyToSymbol(g_spec_to_rgb, m, sizeof(m));
+  cudaMemcpyToSymbol(g_smits, smits, sizeof(smits));
 }
 
 #include "tt_pt2.cuh"
