@@ -305,14 +305,78 @@ __global__ void k_write_nodes(int first, int count, uint32_t n, const Aabb* node
   }
 }
 
+// Scenes of at least this many primitives get byte boxes in their 4-wide nodes: below, the
+// nodes and primitives stay in the L1 whatever their format (closest and any hit measured
+// 2-6 % slower with byte boxes in rooms of 20-40 triangles; 8-10 % faster on the terrain).
+constexpr uint32_t kNode4BytesMin = 16384;
+
+// Writes a 4-wide node of m children with float boxes (layout in tt_build.h).
+__device__ void write_node4_float(float4* d, const Aabb* box, const int* ref, int m) {
+  const float inf = INFINITY;
+  float v[6][4];
+  int rf[4];
+  for (int j = 0; j < 4; ++j) {
+    const Aabb b = j < m ? box[j] : Aabb{make_float3(inf, inf, inf), make_float3(-inf, -inf, -inf)};
+    v[0][j] = b.lo.x;
+    v[1][j] = b.hi.x;
+    v[2][j] = b.lo.y;
+    v[3][j] = b.hi.y;
+    v[4][j] = b.lo.z;
+    v[5][j] = b.hi.z;
+    rf[j] = j < m ? ref[j] : 0x7fffffff;
+  }
+  for (int k = 0; k < 6; ++k) d[k] = make_float4(v[k][0], v[k][1], v[k][2], v[k][3]);
+  d[6] = make_float4(__int_as_float(rf[0]), __int_as_float(rf[1]), __int_as_float(rf[2]), __int_as_float(rf[3]));
+  d[7] = make_float4(0.f, 0.f, 0.f, 0.f);
+}
+
+// Writes a 4-wide node of m children with byte boxes (layout in tt_build.h).  Per axis the grid's step is
+// 1/253 of the children's extent (at least 2^-22 of the coordinates, so that a step is never
+// lost in the float origin) and its origin one step below the lowest plane; lower planes round
+// down and upper planes up with a margin of 1/32 step for the traversal's rounding.  An empty
+// slot has an inverted box (never met) and the first child's reference.
+__device__ void write_node4_bytes(float4* d, const Aabb* box, const int* ref, int m) {
+  float org[3], step[3];
+  unsigned qlo[3], qhi[3];
+  for (int k = 0; k < 3; ++k) {
+    auto lo = [&](int j) { return (double)(k == 0 ? box[j].lo.x : k == 1 ? box[j].lo.y : box[j].lo.z); };
+    auto hi = [&](int j) { return (double)(k == 0 ? box[j].hi.x : k == 1 ? box[j].hi.y : box[j].hi.z); };
+    double a = lo(0), b = hi(0);
+    for (int j = 1; j < m; ++j) {
+      a = fmin(a, lo(j));
+      b = fmax(b, hi(j));
+    }
+    const double s = fmax(fmax((b - a) / 253.0, fmax(fabs(a), fabs(b)) * 2.384185791015625e-07), 1e-30);
+    step[k] = __double2float_ru(s);
+    org[k] = __double2float_rd(a - (double)step[k]);
+    qlo[k] = qhi[k] = 0u;
+    for (int j = 0; j < 4; ++j) {
+      unsigned l = 255u, h = 0u;
+      if (j < m) {
+        l = (unsigned)fmin(255.0, fmax(0.0, floor((lo(j) - org[k]) / step[k] - 0.03125)));
+        h = (unsigned)fmin(255.0, fmax(0.0, ceil((hi(j) - org[k]) / step[k] + 0.03125)));
+      }
+      qlo[k] |= l << (8 * j);
+      qhi[k] |= h << (8 * j);
+    }
+  }
+  d[0] = make_float4(org[0], org[1], org[2], step[0]);
+  d[1] = make_float4(step[1], step[2], __uint_as_float(qlo[0]), __uint_as_float(qlo[1]));
+  d[2] = make_float4(__uint_as_float(qlo[2]), __uint_as_float(qhi[0]), __uint_as_float(qhi[1]), __uint_as_float(qhi[2]));
+  d[3] = make_float4(__int_as_float(ref[0]), __int_as_float(ref[m > 1 ? 1 : 0]), __int_as_float(ref[m > 2 ? 2 : 0]),
+                     __int_as_float(ref[m > 3 ? 3 : 0]));
+}
+
 // 4-wide layout, built top down one level at a time: a 4-wide node starts from a binary
 // inner node's two children and, while it has fewer than four, replaces the inner child of
 // the largest surface area by that child's two children (the usual collapse of a binary
 // tree into a wide one); its remaining inner children become the next level's 4-wide
-// nodes, numbered by an atomic counter.  frontier: (binary node, 4-wide index) pairs.
-__global__ void k_collapse4(const int2* frontier, int nfront, uint32_t n, const Aabb* node_box, const int* left,
+// nodes, numbered by an atomic counter.  frontier: (binary node,
+// 4-wide index, stack entries a traversal may hold when it reaches the node).
+__global__ void k_collapse4(const int4* frontier, int nfront, uint32_t n, const Aabb* node_box, const int* left,
                             const int* right, const int* size, const int* offset, const unsigned char* emit,
-                            const int* index, int* counter, int2* next, int* nnext, float4* nodes4) {
+                            const int* index, int* counter, int4* next, int* nnext, int* stack_need, int bytes,
+                            float4* nodes4) {
   constexpr int kEmpty = 0x7fffffff;
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nfront; t += gridDim.x * blockDim.x) {
     const int k = frontier[t].x, i4 = frontier[t].y;
@@ -338,47 +402,27 @@ __global__ void k_collapse4(const int2* frontier, int nfront, uint32_t n, const 
     }
     Aabb box[4];
     int ref[4];
-    for (int j = 0; j < 4; ++j) {
-      if (j >= m) {
-        box[j] = Aabb{make_float3(INFINITY, INFINITY, INFINITY), make_float3(-INFINITY, -INFINITY, -INFINITY)};
-        ref[j] = kEmpty;
-        continue;
-      }
+    for (int j = 0; j < m; ++j) {
       const int c = slot[j];
       box[j] = node_box[c];
       if (c >= (int)n && emit[c]) {
         const int j4 = atomicAdd(counter, 1);
-        next[atomicAdd(nnext, 1)] = make_int2(c, j4);
+        next[atomicAdd(nnext, 1)] = make_int4(c, j4, frontier[t].z + m - 1, 0);
         ref[j] = j4;
       } else {
         ref[j] = child_ref(c, n, size, offset, emit, index);
       }
     }
-    float4* d = nodes4 + 8 * (size_t)i4;
-    d[0] = make_float4(box[0].lo.x, box[1].lo.x, box[2].lo.x, box[3].lo.x);
-    d[1] = make_float4(box[0].hi.x, box[1].hi.x, box[2].hi.x, box[3].hi.x);
-    d[2] = make_float4(box[0].lo.y, box[1].lo.y, box[2].lo.y, box[3].lo.y);
-    d[3] = make_float4(box[0].hi.y, box[1].hi.y, box[2].hi.y, box[3].hi.y);
-    d[4] = make_float4(box[0].lo.z, box[1].lo.z, box[2].lo.z, box[3].lo.z);
-    d[5] = make_float4(box[0].hi.z, box[1].hi.z, box[2].hi.z, box[3].hi.z);
-    d[6] = make_float4(__int_as_float(ref[0]), __int_as_float(ref[1]), __int_as_float(ref[2]), __int_as_float(ref[3]));
-    d[7] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (bytes) write_node4_bytes(nodes4 + 4 * (size_t)i4, box, ref, m);
+    else write_node4_float(nodes4 + 8 * (size_t)i4, box, ref, m);
+    atomicMax(stack_need, frontier[t].z + 4);
   }
 }
 // 4-wide root of a tree whose root is a leaf: one slot with the leaf.
 __global__ void k_leaf_root4(const Aabb* node_box, int root, int count, float4* nodes4) {
-  const Aabb a = node_box[root];
-  const float inf = INFINITY;
-  nodes4[0] = make_float4(a.lo.x, inf, inf, inf);
-  nodes4[1] = make_float4(a.hi.x, -inf, -inf, -inf);
-  nodes4[2] = make_float4(a.lo.y, inf, inf, inf);
-  nodes4[3] = make_float4(a.hi.y, -inf, -inf, -inf);
-  nodes4[4] = make_float4(a.lo.z, inf, inf, inf);
-  nodes4[5] = make_float4(a.hi.z, -inf, -inf, -inf);
-  const int e = 0x7fffffff;
-  nodes4[6] = make_float4(__int_as_float(~(int)(unsigned)(count - 1)), __int_as_float(e), __int_as_float(e),
-                          __int_as_float(e));
-  nodes4[7] = make_float4(0.f, 0.f, 0.f, 0.f);
+  const Aabb box = node_box[root];
+  const int ref = ~(int)(unsigned)(count - 1);
+  write_node4_float(nodes4, &box, &ref, 1);
 }
 
 // Root handling for trees whose root is a leaf: one node with the leaf as child 0 and an
@@ -581,11 +625,13 @@ bool device_build_bvh2(const BuildInput& in, const uint32_t* set, uint32_t n, De
   // The 4-wide nodes are at most the emitted binary nodes (each 4-wide node replaces at
   // least one); the actual count comes from the collapse.
   const int cap4 = root_emit ? std::max(1, emitted) : 1;
+  out->nodes4_bytes = root_emit && n >= kNode4BytesMin ? 1 : 0;
+  const size_t f4 = out->nodes4_bytes ? 4 : 8;  // float4 per 4-wide node
   if (!ok(pool_malloc((void**)&out->nodes, 4 * sizeof(float4) * (size_t)num_nodes, st), "allocation") ||
       !ok(pool_malloc((void**)&out->tris, 3 * sizeof(float4) * (size_t)n, st), "allocation") ||
-      !ok(pool_malloc((void**)&out->nodes4, 8 * sizeof(float4) * (size_t)cap4, st), "allocation"))
+      !ok(pool_malloc((void**)&out->nodes4, f4 * sizeof(float4) * (size_t)cap4, st), "allocation"))
     return false;
-  int num4 = 1;
+  int num4 = 1, need4 = 0;
   // The root is a leaf when the whole tree collapses (or n == 1): its subtree starts at 0.
   if (!root_emit) {
     cudaMemsetAsync(offset + root, 0, sizeof(int), st);
@@ -595,34 +641,40 @@ bool device_build_bvh2(const BuildInput& in, const uint32_t* set, uint32_t n, De
     for (const auto& r : ranges)
       k_write_nodes<<<grid_for(r.second), kThreads, 0, st>>>(r.first, r.second, n, node_box, left, right, size, offset,
                                                               emit, index, out->nodes);
-    int2* front[2] = {sc.alloc<int2>(cap4), sc.alloc<int2>(cap4)};
-    int* counts = sc.alloc<int>(2);  // [0] 4-wide nodes numbered, [1] next level's size
+    int4* front[2] = {sc.alloc<int4>(cap4), sc.alloc<int4>(cap4)};
+    int* counts = sc.alloc<int>(3);  // [0] 4-wide nodes numbered, [1] next level's size, [2] stack entries needed
     if (!front[0] || !front[1] || !counts) return fail("out of device memory");
-    hb[8] = root;  // the first front: (root, 0); counts: {1, 0}
-    hb[9] = 0;
-    hb[10] = 1;
-    hb[11] = 0;
-    cudaMemcpyAsync(front[0], &hb[8], sizeof(int2), cudaMemcpyHostToDevice, st);
-    cudaMemcpyAsync(counts, &hb[10], 2 * sizeof(int), cudaMemcpyHostToDevice, st);
+    const int first[7] = {root, 0, 0, 0, 1, 0, 0};  // the first front: (root, 0); counts: {1, 0, 0}
+    std::copy(first, first + 7, hb + 8);
+    cudaMemcpyAsync(front[0], &hb[8], sizeof(int4), cudaMemcpyHostToDevice, st);
+    cudaMemcpyAsync(counts, &hb[12], 3 * sizeof(int), cudaMemcpyHostToDevice, st);
     int nfront = 1;
     for (int level = 0; nfront > 0 && level < 64; ++level) {
       cudaMemsetAsync(counts + 1, 0, sizeof(int), st);
       k_collapse4<<<grid_for(nfront), kThreads, 0, st>>>(front[level & 1], nfront, n, node_box, left, right, size,
                                                           offset, emit, index, counts, front[(level + 1) & 1],
-                                                          counts + 1, out->nodes4);
-      int* c2 = &hb[12];
-      cudaMemcpyAsync(c2, counts, 2 * sizeof(int), cudaMemcpyDeviceToHost, st);
+                                                          counts + 1, counts + 2, out->nodes4_bytes, out->nodes4);
+      int* c2 = &hb[16];
+      cudaMemcpyAsync(c2, counts, 3 * sizeof(int), cudaMemcpyDeviceToHost, st);
       if (!ok(cudaStreamSynchronize(st), "4-wide collapse")) return false;
       nfront = c2[1];
       num4 = c2[0];
+      need4 = c2[2];
     }
     if (nfront > 0) return fail("4-wide collapse deeper than 64 levels");
-    // Keep the nodes in a buffer of their exact size (the collapse wrote into an upper bound).
-    float4* exact = nullptr;
-    if (!ok(pool_malloc((void**)&exact, 8 * sizeof(float4) * (size_t)num4, st), "allocation")) return false;
-    cudaMemcpyAsync(exact, out->nodes4, 8 * sizeof(float4) * (size_t)num4, cudaMemcpyDeviceToDevice, st);
-    pool_free(out->nodes4, st);
-    out->nodes4 = exact;
+    if (need4 > BVH_STACK) {
+      // A path of the 4-wide tree could push more than the traversal's stack holds: the
+      // binary tree, whose depth the caller checks, serves all rays.
+      pool_free(out->nodes4, st);
+      out->nodes4 = nullptr;
+    } else {
+      // Keep the nodes in a buffer of their exact size (the collapse wrote into an upper bound).
+      float4* exact = nullptr;
+      if (!ok(pool_malloc((void**)&exact, f4 * sizeof(float4) * (size_t)num4, st), "allocation")) return false;
+      cudaMemcpyAsync(exact, out->nodes4, f4 * sizeof(float4) * (size_t)num4, cudaMemcpyDeviceToDevice, st);
+      pool_free(out->nodes4, st);
+      out->nodes4 = exact;
+    }
   }
   k_write_slots<<<grid_for(n), kThreads, 0, st>>>(in, set, left, offset, n, out->tris);
   if (!ok(cudaStreamSynchronize(st), "emission") || !ok(cudaGetLastError(), "kernels")) return false;

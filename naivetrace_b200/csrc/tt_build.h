@@ -27,11 +27,16 @@ struct DeviceBvh {
   uint32_t num_nodes;
   uint32_t max_depth;
   // The same tree with up to four children per node (a binary node's children, the inner
-  // child of the largest surface area replaced by its children until there are four; 8
-  // float4: lo.x[4], hi.x[4], lo.y[4], hi.y[4], lo.z[4], hi.z[4], int4 references (inner
-  // node, leaf reference as in the binary layout, or 0x7fffffff for an empty slot with an
-  // empty box), padding; the root is node 0), from the memory pool.
+  // child of the largest surface area replaced by its children until there are four).
+  // References: inner node, or leaf reference as in the binary layout.  The root is node 0.
+  // Float boxes (nodes4_bytes = 0), 8 float4 per node: lo.x[4], hi.x[4], lo.y[4], hi.y[4],
+  // lo.z[4], hi.z[4], four references (0x7fffffff and an empty box for an empty slot), padding.
+  // Byte boxes (nodes4_bytes = 1), 4 float4 per node as 16 words: grid origin xyz, grid step
+  // xyz, the children's lower plane bytes x, y, z (child j in byte j), their upper plane bytes
+  // x, y, z, four references (an empty slot has an inverted box and the first child's
+  // reference); plane = origin + byte x step.
   float4* nodes4;
+  int nodes4_bytes;
   uint32_t num_nodes4;
 };
 

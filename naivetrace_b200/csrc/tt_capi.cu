@@ -300,6 +300,7 @@ struct tt_ctx {
     bool ready = false;
     const float4* nodes = nullptr;
     const float4* nodes4 = nullptr;
+    int nodes4_bytes = 0;
     const uint4* nodes8 = nullptr;
     const float4* tris = nullptr;
     const float4* vnodes = nullptr;
@@ -646,6 +647,7 @@ static void save_layout(tt_ctx* c) {
   L.ready = true;
   L.nodes = c->dev.nodes;
   L.nodes4 = c->dev.nodes4;
+  L.nodes4_bytes = c->dev.nodes4_bytes;
   L.nodes8 = c->dev.nodes8;
   L.tris = c->dev.tris;
   L.vnodes = c->dev.vnodes;
@@ -689,6 +691,7 @@ static tt_status use_layout(tt_ctx* c, bool wide) {
   c->dev.wide = wide ? 1 : 0;
   c->dev.nodes = L.nodes;
   c->dev.nodes4 = L.nodes4;
+  c->dev.nodes4_bytes = L.nodes4_bytes;
   c->dev.nodes8 = L.nodes8;
   c->dev.tris = L.tris;
   c->dev.vnodes = L.vnodes;
@@ -891,11 +894,12 @@ tt_status tt_upload_scene(tt_ctx* c) {
     s.vnodes = vb.nodes;
     s.vtris = vb.tris;
     if (sb.nodes4 && !binary_only) {
-      // Closest hit runs on the 4-wide nodes; a counted node visit reads 112 bytes (the
-      // eighth float4 of a node is padding).
+      // Surface rays run on the 4-wide nodes (float boxes: a visit reads 112 of a node's 128
+      // bytes, the rest is padding).
       s.nodes4 = sb.nodes4;
+      s.nodes4_bytes = sb.nodes4_bytes;
       c->bvh_nodes = sb.num_nodes4;
-      c->bvh_node_bytes = 112;
+      c->bvh_node_bytes = sb.nodes4_bytes ? 64 : 112;
     }
   } else {
     BvhInput bi{}, vbi{};

@@ -274,6 +274,10 @@ __device__ __forceinline__ bool trace_step(const BvhRef& bvh, TraceState& s, int
   return false;
 }
 
+// Layouts of the surface BVH: binary, four children per node with float boxes or with boxes
+// as bytes on a grid per node, eight children compressed.
+enum { kLayout2 = 2, kLayout4 = 4, kLayout4Bytes = 5, kLayout8 = 8 };
+
 // No node: larger than any node index and not a leaf reference (leaf references are
 // negative, -1 included).
 constexpr int kNoNode = 0x7fffffff;
@@ -379,13 +383,130 @@ __device__ __forceinline__ void trace_ww(const BvhRef& bvh, TraceState& s, int* 
 }
 
 // Traversal of the 4-wide layout (the binary tree collapsed to nodes of up to four
-// children: tt_build.h).  A node's four boxes are tested together (structure of arrays),
-// the hit children sorted by entry distance: the nearest is visited next, the others pushed
-// farthest first.  Closest hit postpones leaves as trace_ww does (speculative while-while);
-// any hit tests a leaf as soon as it reaches it.  Half the binary tree's depth means half
-// the chain of dependent node fetches that bounds the traversal.  (Used for closest hit;
-// the ANY form, leaves tested as soon as reached, measured slower than the binary per-step
-// traversal for shadow rays.)
+// children: tt_build.h).  Two node formats, by scene size (kNode4BytesMin in tt_build.cu):
+//   float boxes, 128 bytes;
+//   byte boxes, 64 bytes: origin and step of a grid per axis and the children's box planes as
+//   bytes on it, rounded outwards.
+// In large scenes the traversal is bound by the L1 (per-lane node reads took 56-63 % of its data
+// pipe at a 48 % hit rate with float boxes) and by issue about equally; byte boxes halve the
+// former (31-37 %).  In small scenes every node hits the L1 and decoding only adds instructions.
+// A plane byte b becomes a float without a conversion: the byte placed in bits 8-15 of the
+// mantissa of 1.0 is 1 + b 2^-15, so t = a + b s / d = fma(1 + b 2^-15, 2^15 s / d, a - 2^15 s / d),
+// a = (p - o) / d, whose rounding (2^-9 of a grid step) the builder's outward margin of 1/32 step
+// covers.  Near and far planes follow the ray's signs: two words per axis swapped instead of a
+// minimum and a maximum per child.  Exit distances are widened by 1 + 2 gamma(3), so the test
+// never loses a box that the ray meets; a box met too many costs its test (1.9 % more nodes and
+// 2.1 % more primitives per ray on the terrain; for the hits see leaf_box_met).  The slab products are packed in pairs
+// (fma.rn.f32x2: terrain x 16 47.0 -> 44.8 ms).  Closest and any hit together with the
+// refill below, terrain 1920x1080 x 64: 185.7 -> 170.6 ms a frame.
+// One 32-byte load (a sector) of two float4 (256-bit global loads, sm_100).
+__device__ __forceinline__ void ldg256(const float4* p, float4& a, float4& b) {
+  asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+      : "l"(p));
+}
+
+// Three-input minimum and maximum (PTX ISA 8.8, sm_100+).
+__device__ __forceinline__ float fmax3(float a, float b, float c) {
+  float d;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+__device__ __forceinline__ float fmin3(float a, float b, float c) {
+  float d;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+
+// Two fused multiply-adds in one instruction (packed f32x2, sm_100).
+__device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;"
+      : "=l"(r)
+      : "l"(*reinterpret_cast<const unsigned long long*>(&a)), "l"(*reinterpret_cast<const unsigned long long*>(&b)),
+        "l"(*reinterpret_cast<const unsigned long long*>(&c)));
+  return *reinterpret_cast<float2*>(&r);
+}
+
+// The children of 4-wide node `node` the ray meets before best_t: entry distances (INFINITY:
+// not met) and references.
+struct Node4 {
+  float d[4];
+  int c[4];
+};
+template <bool BYTES>
+__device__ __forceinline__ Node4 test_node4(const float4* __restrict__ nodes4, const RayPre& r, int node, float tnear,
+                                            float best_t) {
+  Node4 h;
+  if constexpr (!BYTES) {
+    const float4* np = nodes4 + 8 * (size_t)node;
+    float4 p[6];
+    ldg256(np, p[0], p[1]);
+    ldg256(np + 2, p[2], p[3]);
+    ldg256(np + 4, p[4], p[5]);
+    const int4 rf = __ldg(reinterpret_cast<const int4*>(np + 6));
+    h.c[0] = rf.x;
+    h.c[1] = rf.y;
+    h.c[2] = rf.z;
+    h.c[3] = rf.w;
+    const float lim = best_t * 1.0000004f;  // 1 + 2 gamma(3): conservative slabs
+    const float2 ix = make_float2(r.id.x, r.id.x), iy = make_float2(r.id.y, r.id.y), iz = make_float2(r.id.z, r.id.z);
+    const float2 ox = make_float2(-r.ood.x, -r.ood.x), oy = make_float2(-r.ood.y, -r.ood.y),
+                 oz = make_float2(-r.ood.z, -r.ood.z);
+#pragma unroll
+    for (int j = 0; j < 4; j += 2) {
+      const auto two = [&](const float4& v) { return j == 0 ? make_float2(v.x, v.y) : make_float2(v.z, v.w); };
+      const float2 x0 = ffma2(two(p[0]), ix, ox), x1 = ffma2(two(p[1]), ix, ox);
+      const float2 y0 = ffma2(two(p[2]), iy, oy), y1 = ffma2(two(p[3]), iy, oy);
+      const float2 z0 = ffma2(two(p[4]), iz, oz), z1 = ffma2(two(p[5]), iz, oz);
+      const float e0 = fmax3(fminf(x0.x, x1.x), fminf(y0.x, y1.x), fmaxf(fminf(z0.x, z1.x), tnear));
+      const float f0 = fmin3(fmaxf(x0.x, x1.x), fmaxf(y0.x, y1.x), fminf(fmaxf(z0.x, z1.x), lim));
+      const float e1 = fmax3(fminf(x0.y, x1.y), fminf(y0.y, y1.y), fmaxf(fminf(z0.y, z1.y), tnear));
+      const float f1 = fmin3(fmaxf(x0.y, x1.y), fmaxf(y0.y, y1.y), fminf(fmaxf(z0.y, z1.y), lim));
+      h.d[j] = e0 <= f0 && h.c[j] != kNoNode ? e0 : INFINITY;  // empty slots never hit
+      h.d[j + 1] = e1 <= f1 && h.c[j + 1] != kNoNode ? e1 : INFINITY;
+    }
+    return h;
+  }
+  const float4* np = nodes4 + 4 * (size_t)node;
+  float4 n0, n1, n2, n3;
+  ldg256(np, n0, n1);
+  ldg256(np + 2, n2, n3);
+  constexpr float kGrid = 32768.f, kWiden = 1.0000011f;
+  const float sx = n0.w * r.id.x * kGrid, sy = n1.x * r.id.y * kGrid, sz = n1.y * r.id.z * kGrid;
+  const float ax = fmaf(n0.x - r.o.x, r.id.x, -sx), ay = fmaf(n0.y - r.o.y, r.id.y, -sy),
+              az = fmaf(n0.z - r.o.z, r.id.z, -sz);
+  const bool nx = r.id.x < 0.f, ny = r.id.y < 0.f, nz = r.id.z < 0.f;
+  const unsigned lox = __float_as_uint(n1.z), loy = __float_as_uint(n1.w), loz = __float_as_uint(n2.x);
+  const unsigned hix = __float_as_uint(n2.y), hiy = __float_as_uint(n2.z), hiz = __float_as_uint(n2.w);
+  const unsigned px = nx ? hix : lox, fx = nx ? lox : hix;
+  const unsigned py = ny ? hiy : loy, fy = ny ? loy : hiy;
+  const unsigned pz = nz ? hiz : loz, fz = nz ? loz : hiz;
+  h.c[0] = __float_as_int(n3.x);
+  h.c[1] = __float_as_int(n3.y);
+  h.c[2] = __float_as_int(n3.z);
+  h.c[3] = __float_as_int(n3.w);
+  const auto at2 = [&](unsigned w, int j, float s, float a) {
+    return ffma2(make_float2(__uint_as_float(__byte_perm(w, 0x3f800000u, 0x7604u | ((unsigned)j << 4))),
+                             __uint_as_float(__byte_perm(w, 0x3f800000u, 0x7604u | ((unsigned)(j + 1) << 4)))),
+                 make_float2(s, s), make_float2(a, a));
+  };
+#pragma unroll
+  for (int j = 0; j < 4; j += 2) {
+    const float2 ex = at2(px, j, sx, ax), ey = at2(py, j, sy, ay), ez = at2(pz, j, sz, az);
+    const float2 gx = at2(fx, j, sx, ax), gy = at2(fy, j, sy, ay), gz = at2(fz, j, sz, az);
+    const float m0 = fmax3(ex.x, ey.x, fmaxf(ez.x, tnear)), m1 = fmax3(ex.y, ey.y, fmaxf(ez.y, tnear));
+    const float f0 = fmin3(gx.x, gy.x, fminf(gz.x, best_t)), f1 = fmin3(gx.y, gy.y, fminf(gz.y, best_t));
+    h.d[j] = m0 <= f0 * kWiden ? m0 : INFINITY;
+    h.d[j + 1] = m1 <= f1 * kWiden ? m1 : INFINITY;
+  }
+  return h;
+}
+
+// Closest hit: visits 4-wide node `node` and returns the nearest child met (pushing the others
+// farthest first), the stack's top when no child is met, or kNoNode when the stack is empty
+// too.  *overflow is set when the stack is full.  Leaves are postponed by the callers as in
+// trace_ww.
 __device__ __forceinline__ void sort2(float& da, int& ra, float& db, int& rb) {
   if (db < da) {
     const float t = da;
@@ -396,81 +517,140 @@ __device__ __forceinline__ void sort2(float& da, int& ra, float& db, int& rb) {
     rb = u;
   }
 }
-template <bool ANY, bool COUNT, bool SPH>
+template <bool BYTES>
+__device__ __forceinline__ int visit_node4(const float4* __restrict__ nodes4, const RayPre& r, int node, float tnear,
+                                           float best_t, int* stack, int& sp, bool* overflow) {
+  Node4 h = test_node4<BYTES>(nodes4, r, node, tnear, best_t);
+  sort2(h.d[0], h.c[0], h.d[1], h.c[1]);
+  sort2(h.d[2], h.c[2], h.d[3], h.c[3]);
+  sort2(h.d[0], h.c[0], h.d[2], h.c[2]);
+  sort2(h.d[1], h.c[1], h.d[3], h.c[3]);
+  sort2(h.d[1], h.c[1], h.d[2], h.c[2]);
+  if (h.d[0] == INFINITY) return sp > 0 ? stack[--sp] : kNoNode;
+  if (sp + 3 > BVH_STACK) {
+    *overflow = true;
+    return kNoNode;
+  }
+  if (h.d[3] != INFINITY) stack[sp++] = h.c[3];
+  if (h.d[2] != INFINITY) stack[sp++] = h.c[2];
+  if (h.d[1] != INFINITY) stack[sp++] = h.c[1];
+  return h.c[0];
+}
+
+// Any hit (byte boxes): the children in node order (an occluder may lie anywhere: sorting them, fully or the
+// nearest first, measured no faster).
+__device__ __forceinline__ int visit_node4_any(const float4* __restrict__ nodes4, const RayPre& r, int node, float tnear,
+                                               float tfar, int* stack, int& sp, bool* overflow) {
+  const Node4 h = test_node4<true>(nodes4, r, node, tnear, tfar);
+  if (sp + 4 > BVH_STACK) {
+    *overflow = true;
+    return kNoNode;
+  }
+  int next = kNoNode;
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    if (h.d[j] != INFINITY) {
+      if (next != kNoNode) stack[sp++] = h.c[j];
+      else next = h.c[j];
+    }
+  return next != kNoNode ? next : (sp > 0 ? stack[--sp] : kNoNode);
+}
+
+// Byte boxes contain the float boxes, so a traversal of them meets every leaf that the float
+// boxes' traversal meets, and rarely one more: a float slab test can lose a box that the ray
+// touches within rounding of an edge (about one ray in 10^8 on the terrain), and then misses what
+// it holds.  So that hits do not depend on the node format, a hit in a tree of byte boxes counts
+// when the ray meets the leaf's box in the float test (it then meets every box around it, slab
+// distances being monotone in the planes): tested on the primitive's own box, which lies in the
+// leaf's, and only if that fails on the leaf's.
+template <bool SPH>
+__device__ __forceinline__ void slot_box(float4 a, float4 b, float4 c, float3& lo, float3& hi) {
+  lo = f3(fminf(a.x, fminf(b.x, c.x)), fminf(a.y, fminf(b.y, c.y)), fminf(a.z, fminf(b.z, c.z)));
+  hi = f3(fmaxf(a.x, fmaxf(b.x, c.x)), fmaxf(a.y, fmaxf(b.y, c.y)), fmaxf(a.z, fmaxf(b.z, c.z)));
+  if (SPH && __float_as_int(c.w) != 0) {  // as the builders box a sphere
+    lo = f3(nextafterf(a.x - b.x, -INFINITY), nextafterf(a.y - b.x, -INFINITY), nextafterf(a.z - b.x, -INFINITY));
+    hi = f3(nextafterf(a.x + b.x, INFINITY), nextafterf(a.y + b.x, INFINITY), nextafterf(a.z + b.x, INFINITY));
+  }
+}
+__device__ __forceinline__ bool float_box_met(const RayPre& r, float3 lo, float3 hi, float tnear, float best_t) {
+  const float3 ood = f3(__fmul_rn(r.o.x, r.id.x), __fmul_rn(r.o.y, r.id.y), __fmul_rn(r.o.z, r.id.z));
+  const float x0 = fmaf(lo.x, r.id.x, -ood.x), x1 = fmaf(hi.x, r.id.x, -ood.x);
+  const float y0 = fmaf(lo.y, r.id.y, -ood.y), y1 = fmaf(hi.y, r.id.y, -ood.y);
+  const float z0 = fmaf(lo.z, r.id.z, -ood.z), z1 = fmaf(hi.z, r.id.z, -ood.z);
+  const float tmin = fmaxf(fmaxf(fminf(x0, x1), fminf(y0, y1)), fmaxf(fminf(z0, z1), tnear));
+  const float tmax = fminf(fminf(fmaxf(x0, x1), fmaxf(y0, y1)), fminf(fmaxf(z0, z1), best_t * 1.0000004f));
+  return tmin <= tmax;
+}
+template <bool SPH>
+__device__ __forceinline__ bool leaf_box_met(const float4* __restrict__ tris, const RayPre& r, int start, int count,
+                                             float4 a, float4 b, float4 c, float tnear, float best_t) {
+  float3 lo, hi;
+  slot_box<SPH>(a, b, c, lo, hi);
+  if (float_box_met(r, lo, hi, tnear, best_t)) return true;
+#pragma unroll 1
+  for (int i = start; i < start + count; ++i) {
+    float3 l, h;
+    slot_box<SPH>(__ldg(&tris[3 * i]), __ldg(&tris[3 * i + 1]), __ldg(&tris[3 * i + 2]), l, h);
+    lo = f3(fminf(lo.x, l.x), fminf(lo.y, l.y), fminf(lo.z, l.z));
+    hi = f3(fmaxf(hi.x, h.x), fmaxf(hi.y, h.y), fmaxf(hi.z, h.z));
+  }
+  return float_box_met(r, lo, hi, tnear, best_t);
+}
+
+// Tests the primitives of leaf reference `leaf` for a closer hit (ANY: returns true at the
+// first hit); BYTES: the leaf of a tree with byte boxes.
+template <bool ANY, bool BYTES, bool COUNT, bool SPH>
+__device__ __forceinline__ bool test_leaf(const float4* __restrict__ tris, const RayPre& r, int leaf, float tnear,
+                                          float& best_t, int& best, int& best_prim, float& b1o, float& b2o,
+                                          TraceCounters* cnt, bool check = true) {
+  const unsigned v = ~(unsigned)leaf;
+  const int start = (int)(v >> 3), count = (int)(v & 7u) + 1;
+  for (int i = start; i < start + count; ++i) {
+    const float4 a = __ldg(&tris[3 * i]);
+    const float4 b = __ldg(&tris[3 * i + 1]);
+    const float4 cc = __ldg(&tris[3 * i + 2]);
+    if (COUNT) cnt->tris++;
+    float t, b1 = 0.f, b2 = 0.f;
+    bool hit;
+    if (SPH && __float_as_int(cc.w) != 0) hit = intersect_sphere(r, a, b, tnear, best_t, &t);
+    else hit = intersect_tri(r, xyz(a), xyz(b), xyz(cc), tnear, best_t, &t, &b1, &b2);
+    if (hit && (ANY || closer(t, __float_as_int(a.w), best_t, best_prim)) &&
+        (!BYTES || !check || leaf_box_met<SPH>(tris, r, start, count, a, b, cc, tnear, best_t))) {
+      best = i;
+      best_prim = __float_as_int(a.w);
+      best_t = t;
+      b1o = b1;
+      b2o = b2;
+      if (ANY) return true;
+    }
+  }
+  return false;
+}
+
+template <bool BYTES, bool COUNT, bool SPH>
 __device__ __forceinline__ void trace4(const float4* __restrict__ nodes4, const float4* __restrict__ tris,
                                        TraceState& s, int* stack, unsigned int* err, TraceCounters* cnt) {
-  const RayPre& r = s.r;
   int cur = 0;
   int leaf = kNoNode;
   int sp = 0;
   while (cur != kNoNode || leaf != kNoNode) {
     while ((unsigned)cur < (unsigned)kNoNode) {
-      const float4* np = nodes4 + 8 * (size_t)cur;
-      const float4 lx = __ldg(np), hx = __ldg(np + 1), ly = __ldg(np + 2), hy = __ldg(np + 3);
-      const float4 lz = __ldg(np + 4), hz = __ldg(np + 5);
-      const int4 rf = __ldg(reinterpret_cast<const int4*>(np + 6));
+      bool overflow = false;
+      cur = visit_node4<BYTES>(nodes4, s.r, cur, s.tnear, s.best_t, stack, sp, &overflow);
       if (COUNT) cnt->nodes++;
-      const float lim = s.best_t * 1.0000004f;  // 1 + 2 gamma(3): conservative slabs
-      const float lxs[4] = {lx.x, lx.y, lx.z, lx.w}, hxs[4] = {hx.x, hx.y, hx.z, hx.w};
-      const float lys[4] = {ly.x, ly.y, ly.z, ly.w}, hys[4] = {hy.x, hy.y, hy.z, hy.w};
-      const float lzs[4] = {lz.x, lz.y, lz.z, lz.w}, hzs[4] = {hz.x, hz.y, hz.z, hz.w};
-      float d[4];
-      int c[4] = {rf.x, rf.y, rf.z, rf.w};
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float tx0 = fmaf(lxs[j], r.id.x, -r.ood.x), tx1 = fmaf(hxs[j], r.id.x, -r.ood.x);
-        const float ty0 = fmaf(lys[j], r.id.y, -r.ood.y), ty1 = fmaf(hys[j], r.id.y, -r.ood.y);
-        const float tz0 = fmaf(lzs[j], r.id.z, -r.ood.z), tz1 = fmaf(hzs[j], r.id.z, -r.ood.z);
-        const float tmin = fmaxf(fmaxf(fminf(tx0, tx1), fminf(ty0, ty1)), fmaxf(fminf(tz0, tz1), s.tnear));
-        const float tmax = fminf(fminf(fmaxf(tx0, tx1), fmaxf(ty0, ty1)), fminf(fmaxf(tz0, tz1), lim));
-        d[j] = (tmin <= tmax && c[j] != kNoNode) ? tmin : INFINITY;  // empty slots never hit
-      }
-      sort2(d[0], c[0], d[1], c[1]);
-      sort2(d[2], c[2], d[3], c[3]);
-      sort2(d[0], c[0], d[2], c[2]);
-      sort2(d[1], c[1], d[3], c[3]);
-      sort2(d[1], c[1], d[2], c[2]);
-      if (d[0] == INFINITY) {
-        cur = sp > 0 ? stack[--sp] : kNoNode;
-      } else {
-        if (sp + 3 > BVH_STACK) {
-          atomicOr(err, ERR_STACK);
-          s.best = -1;
-          return;
-        }
-        if (d[3] != INFINITY) stack[sp++] = c[3];
-        if (d[2] != INFINITY) stack[sp++] = c[2];
-        if (d[1] != INFINITY) stack[sp++] = c[1];
-        cur = c[0];
+      if (overflow) {
+        atomicOr(err, ERR_STACK);
+        s.best = -1;
+        return;
       }
       if (cur < 0 && leaf == kNoNode) {
         leaf = cur;
         cur = sp > 0 ? stack[--sp] : kNoNode;
-        if (ANY) break;
       }
-      if (!ANY && !__any_sync(__activemask(), leaf == kNoNode)) break;
+      if (!__any_sync(__activemask(), leaf == kNoNode)) break;
     }
     while (leaf != kNoNode) {
-      const unsigned v = ~(unsigned)leaf;
-      const int start = (int)(v >> 3), count = (int)(v & 7u) + 1;
-      for (int i = start; i < start + count; ++i) {
-        const float4 a = __ldg(&tris[3 * i]);
-        const float4 b = __ldg(&tris[3 * i + 1]);
-        const float4 cc = __ldg(&tris[3 * i + 2]);
-        if (COUNT) cnt->tris++;
-        float t, b1 = 0.f, b2 = 0.f;
-        bool hit;
-        if (SPH && __float_as_int(cc.w) != 0) hit = intersect_sphere(r, a, b, s.tnear, s.best_t, &t);
-        else hit = intersect_tri(r, xyz(a), xyz(b), xyz(cc), s.tnear, s.best_t, &t, &b1, &b2);
-        if (hit && (ANY || closer(t, __float_as_int(a.w), s.best_t, s.best_prim))) {
-          s.best = i;
-          s.best_prim = __float_as_int(a.w);
-          s.best_t = t;
-          s.b1 = b1;
-          s.b2 = b2;
-          if (ANY) return;
-        }
-      }
+      test_leaf<false, BYTES, COUNT, SPH>(tris, s.r, leaf, s.tnear, s.best_t, s.best, s.best_prim, s.b1, s.b2, cnt);
       leaf = kNoNode;
       if (cur < 0) {
         leaf = cur;
@@ -478,6 +658,24 @@ __device__ __forceinline__ void trace4(const float4* __restrict__ nodes4, const 
       }
     }
   }
+}
+
+// One any-hit step on the 4-wide layout with byte boxes: a node or a leaf, so that a lane meets its first
+// occluder as early as the tree order allows.  Returns true when the ray is finished.
+template <bool COUNT, bool SPH>
+__device__ __forceinline__ bool any_step4(const DevScene& sc, TraceState& s, int* stack, unsigned int* err,
+                                          TraceCounters* cnt) {
+  if (s.cur >= 0) {
+    bool overflow = false;
+    s.cur = visit_node4_any(sc.nodes4, s.r, s.cur, s.tnear, s.best_t, stack, s.sp, &overflow);
+    if (COUNT) cnt->nodes++;
+    if (overflow) atomicOr(err, ERR_STACK);
+  } else {
+    if (test_leaf<true, true, COUNT, SPH>(sc.tris, s.r, s.cur, s.tnear, s.best_t, s.best, s.best_prim, s.b1, s.b2, cnt))
+      return true;
+    s.cur = s.sp > 0 ? stack[--s.sp] : kNoNode;
+  }
+  return s.cur == kNoNode;
 }
 
 // Recomputes the distance of the closest hit from the plane equation in double precision
@@ -495,6 +693,162 @@ __device__ __forceinline__ float refine_t(const float4* tris, const RayPre& r, i
 }
 
 // ----------------------------------------------------------------------------------------
+// Traversal of a queue of rays with refilled lanes.  Rays of one warp need very different
+// numbers of steps: with one ray per lane until the longest is done, a warp instruction of
+// the closest-hit kernel served 17.6 lanes on camera rays and 10.9 on the first bounce, 7.7 in
+// the any-hit kernel (terrain, 1920x1080).  Here a warp writes out its finished rays and takes
+// new ones as soon as kRefillClosest (kRefillAny) lanes are idle (dynamic fetch, Aila and Laine
+// 2009), checked once per round of inner nodes and leaves.  (Refilling after every step with any idle lane
+// measured 20 % slower than not refilling: a refill costs the warp a ray set-up and the
+// write-out whatever the number of lanes it serves.)
+// Terrain x 16 with byte boxes: 48.2 ms without refill, 44.7 with it at 8-12 idle lanes, 47.8 at 4;
+// any hit is flat from 8 to 20.  In scenes of a few dozen primitives it measured 4-8 % slower (the
+// rays end together), so float-box scenes run one ray per lane.
+//
+// A warp's share of the queue is every `warps`-th chunk of 32 entries: no counter in memory,
+// neighbouring rays together.
+constexpr int kRefillClosest = 12, kRefillAny = 20;  // idle lanes that end the traversal rounds
+struct WarpShare {
+  unsigned n, warp, warps, taken;
+  __device__ __forceinline__ explicit WarpShare(int count)
+      : n((unsigned)count), warp((blockIdx.x * blockDim.x + threadIdx.x) >> 5), warps((gridDim.x * blockDim.x) >> 5),
+        taken(0u) {}
+  __device__ __forceinline__ unsigned index(unsigned lin) const {
+    return ((lin >> 5) * warps + warp) * 32u + (lin & 31u);
+  }
+  __device__ __forceinline__ bool more() const { return index(taken) < n; }
+};
+
+// Closest hits of the rays 0 .. n-1 of `job` on the 4-wide layout.  job.load(k, ...) gives ray
+// k, job.store(k, r, slot, t, b1, b2) takes its result (slot -1: no hit).  All 32 lanes of
+// every warp of the grid take part.
+template <bool COUNT, bool SPH, class Job>
+__device__ __forceinline__ void closest_queue4(const DevScene& sc, const Job& job, int n, unsigned int* err,
+                                               TraceCounters* cnt) {
+  const unsigned lane = threadIdx.x & 31u;
+  WarpShare share(n);
+  int stack[BVH_STACK];
+  RayPre r;
+  float tnear = 0.f, best_t = 0.f, b1 = 0.f, b2 = 0.f;
+  int best = -1, best_prim = 0, cur = kNoNode, leaf = kNoNode, sp = 0, ray = -1;
+  bool check = false;  // the ray's hits are tested against the leaf's float box
+  for (;;) {
+    bool idle = cur == kNoNode && leaf == kNoNode;
+    if (idle && ray >= 0) {
+      bool met = true;
+      if (best >= 0 && !check) {
+        float3 lo, hi;
+        slot_box<SPH>(__ldg(&sc.tris[3 * best]), __ldg(&sc.tris[3 * best + 1]), __ldg(&sc.tris[3 * best + 2]), lo, hi);
+        met = float_box_met(r, lo, hi, tnear, best_t);
+      }
+      if (met) {
+        job.store(ray, r, best, best_t, b1, b2);
+        ray = -1;
+      } else {  // rare: once more with the test at every hit
+        float3 o, d;
+        job.load(ray, o, d, tnear, best_t);
+        best = -1;
+        best_prim = 0x7fffffff;
+        b1 = b2 = 0.f;
+        cur = 0;
+        sp = 0;
+        idle = false;
+        check = true;
+      }
+    }
+    const unsigned free = __ballot_sync(0xffffffffu, idle);
+    if (share.more()) {
+      if (idle) {
+        const unsigned k = share.index(share.taken + __popc(free & ((1u << lane) - 1u)));
+        if (k < share.n) {
+          ray = (int)k;
+          float3 o, d;
+          job.load(ray, o, d, tnear, best_t);
+          r = prepare_ray(o, d);
+          best = -1;
+          best_prim = 0x7fffffff;
+          b1 = b2 = 0.f;
+          cur = 0;
+          sp = 0;
+          idle = false;
+          check = false;
+        }
+      }
+      share.taken += __popc(free);
+    } else if (free == 0xffffffffu) {
+      break;
+    }
+    const int enough = share.more() ? kRefillClosest : 32;
+    do {
+      while ((unsigned)cur < (unsigned)kNoNode) {
+        bool overflow = false;
+        cur = visit_node4<true>(sc.nodes4, r, cur, tnear, best_t, stack, sp, &overflow);
+        if (COUNT) cnt->nodes++;
+        if (overflow) {
+          atomicOr(err, ERR_STACK);
+          best = -1;
+          leaf = kNoNode;
+          break;
+        }
+        if (cur < 0 && leaf == kNoNode) {
+          leaf = cur;
+          cur = sp > 0 ? stack[--sp] : kNoNode;
+        }
+        if (!__any_sync(__activemask(), leaf == kNoNode)) break;
+      }
+      while (leaf != kNoNode) {
+        test_leaf<false, true, COUNT, SPH>(sc.tris, r, leaf, tnear, best_t, best, best_prim, b1, b2, cnt, check);
+        leaf = kNoNode;
+        if (cur < 0) {
+          leaf = cur;
+          cur = sp > 0 ? stack[--sp] : kNoNode;
+        }
+      }
+      idle = cur == kNoNode;
+    } while (__popc(__ballot_sync(0xffffffffu, idle)) < enough);
+  }
+}
+
+// Any hit of the rays 0 .. n-1 of `job` on the 4-wide layout.  job.store(k, r, slot).
+template <bool COUNT, bool SPH, class Job>
+__device__ __forceinline__ void any_queue4(const DevScene& sc, const Job& job, int n, unsigned int* err,
+                                           TraceCounters* cnt) {
+  const unsigned lane = threadIdx.x & 31u;
+  WarpShare share(n);
+  int stack[BVH_STACK];
+  TraceState s;
+  int ray = -1;
+  bool idle = true;
+  for (;;) {
+    if (idle && ray >= 0) {
+      job.store(ray, s.r, s.best);
+      ray = -1;
+    }
+    const unsigned free = __ballot_sync(0xffffffffu, idle);
+    if (share.more()) {
+      if (idle) {
+        const unsigned k = share.index(share.taken + __popc(free & ((1u << lane) - 1u)));
+        if (k < share.n) {
+          ray = (int)k;
+          float3 o, d;
+          float tnear, tfar;
+          job.load(ray, o, d, tnear, tfar);
+          trace_init(s, o, d, tnear, tfar);
+          idle = false;
+        }
+      }
+      share.taken += __popc(free);
+    } else if (free == 0xffffffffu) {
+      break;
+    }
+    const int enough = share.more() ? kRefillAny : 32;
+    do {
+      if (!idle) idle = any_step4<COUNT, SPH>(sc, s, stack, err, cnt);
+    } while (__popc(__ballot_sync(0xffffffffu, idle)) < enough);
+  }
+}
+
+// ----------------------------------------------------------------------------------------
 // 8-wide BVH traversal (layout in tt_bvh.h), after the compressed wide BVH of Ylitie, Karras
 // and Laine (2017): one 80-byte node gives the quantised boxes of eight children; hit
 // inner children form a "node group" (first child index, inner mask, hit bits in
@@ -508,18 +862,6 @@ __device__ __forceinline__ unsigned permute8(unsigned m, unsigned oct) {
   if (oct & 2u) m = ((m & 0x33u) << 2) | ((m & 0xCCu) >> 2);
   if (oct & 4u) m = ((m & 0x0Fu) << 4) | ((m & 0xF0u) >> 4);
   return m;
-}
-
-// Three-input minimum and maximum (PTX ISA 8.8, sm_100+).
-__device__ __forceinline__ float fmax3(float a, float b, float c) {
-  float d;
-  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
-  return d;
-}
-__device__ __forceinline__ float fmin3(float a, float b, float c) {
-  float d;
-  asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
-  return d;
 }
 
 struct Trace8State {
@@ -634,11 +976,11 @@ __device__ __forceinline__ void trace8_run(const uint4* __restrict__ nodes, cons
   }
 }
 
-// Whole traversal of one ray (batch queries).  Returns the triangle slot or -1.
-template <bool ANY, bool COUNT, bool SPH, bool WIDE>
+// Whole traversal of one ray on layout L.  Returns the primitive slot or -1.
+template <bool ANY, bool COUNT, bool SPH, int L>
 __device__ __forceinline__ int trace(const DevScene& sc, const RayPre& r, float tnear, float tfar, float* t_out,
                                      float* b1_out, float* b2_out, unsigned int* err, TraceCounters* cnt) {
-  if (WIDE) {
+  if constexpr (L == kLayout8) {
     Trace8State s;
     s.tnear = tnear;
     s.best_t = tfar;
@@ -664,14 +1006,15 @@ __device__ __forceinline__ int trace(const DevScene& sc, const RayPre& r, float 
   s.best_prim = 0x7fffffff;
   s.cur = 0;
   s.sp = 0;
-  if (!ANY && sc.nodes4) {
-    // Closest hit on the 4-wide nodes (6 % less closest-hit time than the binary while-while
-    // traversal on the terrain workload).
-    trace4<ANY, COUNT, SPH>(sc.nodes4, sc.tris, s, stack, err, cnt);
-  } else if (ANY) {
+  if constexpr (!ANY && (L == kLayout4 || L == kLayout4Bytes)) {
+    trace4<L == kLayout4Bytes, COUNT, SPH>(sc.nodes4, sc.tris, s, stack, err, cnt);
+  } else if constexpr (L == kLayout4Bytes) {
+    while (!any_step4<COUNT, SPH>(sc, s, stack, err, cnt)) {
+    }
+  } else if constexpr (ANY) {
     // Any hit: one binary node or leaf per step, so that a lane meets its first hit as early
     // as the tree order allows (postponing leaves measured 3.5 % slower for shadow rays, the
-    // 4-wide nodes 7 % slower).
+    // 4-wide nodes with float boxes 2-7 %).
     while (!trace_step<ANY, COUNT, SPH>(bvh, s, stack, err, cnt)) {
     }
   } else {
@@ -1145,41 +1488,38 @@ __host__ __device__ __forceinline__ bool sorted_bounce(const DevScene& sc, const
 // counter addresses).
 struct KeyHistogram {
   int* h;  // kShadeKeys shared ints
-  __device__ void clear() {
+  __device__ void clear() const {
     if (threadIdx.x < kShadeKeys) h[threadIdx.x] = 0;
   }
-  __device__ void add(int key) {
+  __device__ void add(int key) const {
     const unsigned peers = __match_any_sync(__activemask(), key);
     if ((threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(&h[key], __popc(peers));
   }
   // After a __syncthreads that follows every add.
-  __device__ void flush(int* global) {
+  __device__ void flush(int* global) const {
     if (threadIdx.x < kShadeKeys && h[threadIdx.x] != 0) atomicAdd(&global[threadIdx.x], h[threadIdx.x]);
   }
 };
 
-// Closest hit of the queued extension rays, one ray per thread over a grid-stride loop
-// sized to the SM count times the kernel's resident blocks.  (A persistent variant that
-// refilled finished lanes after every traversal step measured 20 % slower.)
-template <bool COUNT, bool SPH, bool WIDE>
-__global__ void __launch_bounds__(256) k_extend(DevScene sc, PathState p, int bounce, unsigned long long* counters) {
-  const int n = *ext_count(p, bounce);
-  const int* q = p.ext_q[bounce & 1];
-  const bool keyed = sc.algo == TT_ALGO_PT && sc.num_media == 0 && sorted_bounce(sc, p, bounce);
-  __shared__ int hist_mem[kShadeKeys];
-  KeyHistogram hist{hist_mem};
-  if (keyed) {
-    hist.clear();
-    __syncthreads();
-  }
-  TraceCounters cnt{0u, 0u};
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+// Closest hit of the queued extension rays: on the 4-wide layout (the default) the queue is
+// traversed with refilled lanes, on the binary and the 8-wide layouts one ray per thread over a
+// grid-stride loop.
+struct ExtendJob {
+  const DevScene& sc;
+  const PathState& p;
+  const int* q;
+  bool keyed;
+  KeyHistogram hist;
+  __device__ __forceinline__ void load(int i, float3& o, float3& d, float& tnear, float& tfar) const {
     const int slot = q[i];
-    const float4 o = p.ray_o[slot], d = p.ray_d[slot];
-    const RayPre r = prepare_ray(xyz(o), xyz(d));
-    float t = 0.f, b1 = 0.f, b2 = 0.f;
-    const int hit = trace<false, COUNT, SPH, WIDE>(sc, r, 0.f, d.w, &t, &b1, &b2, p.err, &cnt);
-    p.hit[slot] = make_float4(t, b1, b2, __int_as_float(hit));
+    const float4 o4 = p.ray_o[slot], d4 = p.ray_d[slot];
+    o = xyz(o4);
+    d = xyz(d4);
+    tnear = 0.f;
+    tfar = d4.w;
+  }
+  __device__ __forceinline__ void put(int i, float t, float b1, float b2, int hit) const {
+    p.hit[q[i]] = make_float4(t, b1, b2, __int_as_float(hit));
     if (keyed) {
       // Material sort, scenes without media: key and count the hit here.
       const int key = hit_key(sc, hit);
@@ -1187,9 +1527,44 @@ __global__ void __launch_bounds__(256) k_extend(DevScene sc, PathState p, int bo
       hist.add(key);
     }
   }
+};
+template <bool SPH>
+struct ExtendStore : ExtendJob {
+  __device__ __forceinline__ explicit ExtendStore(const ExtendJob& j) : ExtendJob(j) {}
+  __device__ __forceinline__ void store(int i, const RayPre& r, int hit, float t, float b1, float b2) const {
+    if (hit < 0) t = b1 = b2 = 0.f;
+    else if (!(SPH && is_sphere_slot(sc.tris, hit))) t = refine_t(sc.tris, r, hit);
+    put(i, t, b1, b2, hit);
+  }
+};
+
+template <bool COUNT, bool SPH, int L>
+__global__ void __launch_bounds__(256) k_extend(DevScene sc, PathState p, int bounce, unsigned long long* counters) {
+  const int n = *ext_count(p, bounce);
+  const bool keyed = sc.algo == TT_ALGO_PT && sc.num_media == 0 && sorted_bounce(sc, p, bounce);
+  __shared__ int hist_mem[kShadeKeys];
+  const ExtendJob job{sc, p, p.ext_q[bounce & 1], keyed, KeyHistogram{hist_mem}};
+  if (keyed) {
+    job.hist.clear();
+    __syncthreads();
+  }
+  TraceCounters cnt{0u, 0u};
+  if constexpr (L == kLayout4Bytes) {
+    closest_queue4<COUNT, SPH>(sc, ExtendStore<SPH>(job), n, p.err, &cnt);
+  } else {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+      float3 o, d;
+      float tnear, tfar;
+      job.load(i, o, d, tnear, tfar);
+      const RayPre r = prepare_ray(o, d);
+      float t = 0.f, b1 = 0.f, b2 = 0.f;
+      const int hit = trace<false, COUNT, SPH, L>(sc, r, tnear, tfar, &t, &b1, &b2, p.err, &cnt);
+      job.put(i, t, b1, b2, hit);
+    }
+  }
   if (keyed) {  // uniform over the grid
     __syncthreads();
-    hist.flush(key_count(p, bounce));
+    job.hist.flush(key_count(p, bounce));
   }
   if (COUNT) {
     atomicAdd(&counters[0], (unsigned long long)cnt.nodes);
@@ -1869,22 +2244,70 @@ __global__ void __launch_bounds__(kTcThreads) k_guide_tc(DevScene sc, PathState 
   tc_teardown(tsm);
 }
 
+// The contribution c of an unoccluded shadow ray: to its path, or (target >= 0, camera-vertex
+// samples) splatted to the pixel it projects to.
+__device__ __forceinline__ void add_unoccluded(const DevScene& sc, const PathState& p, const Framebuffer& fb, int bounce,
+                                               int slot, int target, float3 c) {
+  if (target < 0) {
+    const float4 a = p.accum[slot];
+    p.accum[slot] = make_float4(a.x + c.x, a.y + c.y, a.z + c.z, 0.f);
+    if (sc.guide_record) {
+      // Direct light at the recorded vertex is not radiance along its sampled direction.
+      const float4 r3 = p.grec[(size_t)kRecF4 * slot + 3];
+      if (r3.w != 0.f && __float_as_int(r3.y) == bounce - 1) {
+        const float4 r4 = p.grec[(size_t)kRecF4 * slot + 4];
+        p.grec[(size_t)kRecF4 * slot + 4] = make_float4(r4.x + c.x, r4.y + c.y, r4.z + c.z, 0.f);
+      }
+    }
+  } else {
+    const Lambda l = unpack_lambda(p.meta[slot].y);
+    const float3 rgb = selection_to_rgb(c, l);
+    atomicAdd(&fb.light[3 * target], rgb.x);
+    atomicAdd(&fb.light[3 * target + 1], rgb.y);
+    atomicAdd(&fb.light[3 * target + 2], rgb.z);
+  }
+}
+
+struct ShadowJob {
+  const DevScene& sc;
+  const PathState& p;
+  const Framebuffer& fb;
+  int bounce;
+  __device__ __forceinline__ void load(int i, float3& o, float3& d, float& tnear, float& tfar) const {
+    const int slot = p.sh_q[i];
+    const float4 o4 = p.sh_o[slot], d4 = p.sh_d[slot];
+    o = xyz(o4);
+    d = xyz(d4);
+    tnear = 0.f;
+    tfar = o4.w;
+  }
+  __device__ __forceinline__ void store(int i, const RayPre&, int hit) const {
+    if (hit >= 0) return;
+    const int slot = p.sh_q[i];
+    add_unoccluded(sc, p, fb, bounce, slot, __float_as_int(p.sh_d[slot].w), xyz(p.sh_c[slot]));
+  }
+};
+
 // Occlusion test of the queued shadow rays.  Unoccluded rays add their contribution to
 // the path (or, for camera-vertex samples, splat it to the pixel they project to).  In
 // media scenes the contribution is multiplied by the transmittance through the media
 // between the medium-boundary crossings (TransmittanceEstimate, rendering_util.cxx:40-67)
 // and by the MIS weight that the segment's transmittance pdf factor completes.
-template <bool MEDIA, bool COUNT, bool SPH, bool WIDE>
+template <bool MEDIA, bool COUNT, bool SPH, int L>
 __global__ void __launch_bounds__(256) k_shadow(DevScene sc, PathState p, Framebuffer fb, int bounce,
                                                 unsigned long long* counters) {
   const int n = *sh_count(p, bounce);
   TraceCounters cnt{0u, 0u};
+  constexpr bool WIDE = L == kLayout8;
+  if constexpr (!MEDIA && L == kLayout4Bytes) {
+    any_queue4<COUNT, SPH>(sc, ShadowJob{sc, p, fb, bounce}, n, p.err, &cnt);
+  } else
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const int slot = p.sh_q[i];
     const float4 o = p.sh_o[slot], d = p.sh_d[slot];
     const RayPre r = prepare_ray(xyz(o), xyz(d));
     float t, b1, b2;
-    const int hit = trace<true, COUNT, SPH, WIDE>(sc, r, 0.f, o.w, &t, &b1, &b2, p.err, &cnt);
+    const int hit = trace<true, COUNT, SPH, L>(sc, r, 0.f, o.w, &t, &b1, &b2, p.err, &cnt);
     if (hit >= 0) continue;
     const float4 c4 = p.sh_c[slot];
     float3 c = xyz(c4);
@@ -1922,24 +2345,7 @@ __global__ void __launch_bounds__(256) k_shadow(DevScene sc, PathState p, Frameb
       const float mis = med.x < 0.f ? 1.f : power_heuristic(med.x, med.y * ctr);
       c = mul(c, T) * mis;
     }
-    if (target < 0) {
-      const float4 a = p.accum[slot];
-      p.accum[slot] = make_float4(a.x + c.x, a.y + c.y, a.z + c.z, 0.f);
-      if (sc.guide_record) {
-        // Direct light at the recorded vertex is not radiance along its sampled direction.
-        const float4 r3 = p.grec[(size_t)kRecF4 * slot + 3];
-        if (r3.w != 0.f && __float_as_int(r3.y) == bounce - 1) {
-          const float4 r4 = p.grec[(size_t)kRecF4 * slot + 4];
-          p.grec[(size_t)kRecF4 * slot + 4] = make_float4(r4.x + c.x, r4.y + c.y, r4.z + c.z, 0.f);
-        }
-      }
-    } else {
-      const Lambda l = unpack_lambda(p.meta[slot].y);
-      const float3 rgb = selection_to_rgb(c, l);
-      atomicAdd(&fb.light[3 * target], rgb.x);
-      atomicAdd(&fb.light[3 * target + 1], rgb.y);
-      atomicAdd(&fb.light[3 * target + 2], rgb.z);
-    }
+    add_unoccluded(sc, p, fb, bounce, slot, target, c);
   }
   if (COUNT) {
     atomicAdd(&counters[0], (unsigned long long)cnt.nodes);
@@ -2052,34 +2458,81 @@ __global__ void k_accumulate(Framebuffer fb, double* acc, double* light, int n3)
 
 // ----------------------------------------------------------------------------------------
 // Batch queries and shader sampling for the parity tests.
-template <bool SPH, bool WIDE>
-__global__ void k_intersect_rays(DevScene sc, const float* rays, int n, int* prim, float* t, float* u, float* v,
-                                 unsigned int* err) {
-  TraceCounters cnt{0u, 0u};
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+struct RayJob {
+  const float* rays;
+  __device__ __forceinline__ void load(int i, float3& o, float3& d, float& tnear, float& tfar) const {
     const float* r = rays + 8 * (size_t)i;
-    const RayPre rp = prepare_ray(f3(r[0], r[1], r[2]), f3(r[4], r[5], r[6]));
-    float tt = -1.f, b1 = 0.f, b2 = 0.f;
-    const int slot = trace<false, false, SPH, WIDE>(sc, rp, r[3], r[7], &tt, &b1, &b2, err, &cnt);
+    o = f3(r[0], r[1], r[2]);
+    tnear = r[3];
+    d = f3(r[4], r[5], r[6]);
+    tfar = r[7];
+  }
+};
+template <bool SPH>
+struct IntersectJob : RayJob {
+  const DevScene& sc;
+  int* prim;
+  float *t, *u, *v;
+  __device__ __forceinline__ IntersectJob(const float* rays, const DevScene& sc_, int* prim_, float* t_, float* u_,
+                                          float* v_)
+      : RayJob{rays}, sc(sc_), prim(prim_), t(t_), u(u_), v(v_) {}
+  __device__ __forceinline__ void put(int i, int slot, float tt, float b1, float b2) const {
     prim[i] = slot >= 0 ? __float_as_int(__ldg(&sc.tris[3 * slot]).w) : -1;
     t[i] = slot >= 0 ? tt : -1.f;
     u[i] = b1;
     v[i] = b2;
   }
-}
+  __device__ __forceinline__ void store(int i, const RayPre& r, int slot, float tt, float b1, float b2) const {
+    if (slot < 0) b1 = b2 = 0.f;
+    else if (!(SPH && is_sphere_slot(sc.tris, slot))) tt = refine_t(sc.tris, r, slot);
+    put(i, slot, tt, b1, b2);
+  }
+};
+struct OccludedJob : RayJob {
+  unsigned char* occ;
+  __device__ __forceinline__ OccludedJob(const float* rays, unsigned char* occ_) : RayJob{rays}, occ(occ_) {}
+  __device__ __forceinline__ void store(int i, const RayPre&, int slot) const { occ[i] = slot >= 0 ? 1 : 0; }
+};
 
-template <bool SPH, bool WIDE>
-__global__ void k_occluded_rays(DevScene sc, const float* rays, int n, unsigned char* occ, unsigned int* err) {
+template <bool SPH, int L>
+__global__ void __launch_bounds__(256) k_intersect_rays(DevScene sc, const float* rays, int n, int* prim, float* t,
+                                                        float* u, float* v, unsigned int* err) {
   TraceCounters cnt{0u, 0u};
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const float* r = rays + 8 * (size_t)i;
-    const RayPre rp = prepare_ray(f3(r[0], r[1], r[2]), f3(r[4], r[5], r[6]));
-    float tt, b1, b2;
-    occ[i] = trace<true, false, SPH, WIDE>(sc, rp, r[3], r[7], &tt, &b1, &b2, err, &cnt) >= 0 ? 1 : 0;
+  const IntersectJob<SPH> job(rays, sc, prim, t, u, v);
+  if constexpr (L == kLayout4Bytes) {
+    closest_queue4<false, SPH>(sc, job, n, err, &cnt);
+  } else {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+      float3 o, d;
+      float tnear, tfar;
+      job.load(i, o, d, tnear, tfar);
+      const RayPre rp = prepare_ray(o, d);
+      float tt = -1.f, b1 = 0.f, b2 = 0.f;
+      const int slot = trace<false, false, SPH, L>(sc, rp, tnear, tfar, &tt, &b1, &b2, err, &cnt);
+      job.put(i, slot, tt, b1, b2);
+    }
   }
 }
 
-template <bool SPH, bool WIDE>
+template <bool SPH, int L>
+__global__ void __launch_bounds__(256) k_occluded_rays(DevScene sc, const float* rays, int n, unsigned char* occ,
+                                                       unsigned int* err) {
+  TraceCounters cnt{0u, 0u};
+  const OccludedJob job(rays, occ);
+  if constexpr (L == kLayout4Bytes) {
+    any_queue4<false, SPH>(sc, job, n, err, &cnt);
+  } else {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+      float3 o, d;
+      float tnear, tfar, tt, b1, b2;
+      job.load(i, o, d, tnear, tfar);
+      const RayPre rp = prepare_ray(o, d);
+      job.store(i, rp, trace<true, false, SPH, L>(sc, rp, tnear, tfar, &tt, &b1, &b2, err, &cnt));
+    }
+  }
+}
+
+template <bool SPH, int L>
 __global__ void k_count_rays(DevScene sc, const float* rays, int n, unsigned long long* counters,
                              unsigned int* err) {
   TraceCounters cnt{0u, 0u};
@@ -2087,7 +2540,7 @@ __global__ void k_count_rays(DevScene sc, const float* rays, int n, unsigned lon
     const float* r = rays + 8 * (size_t)i;
     const RayPre rp = prepare_ray(f3(r[0], r[1], r[2]), f3(r[4], r[5], r[6]));
     float tt, b1, b2;
-    trace<false, true, SPH, WIDE>(sc, rp, r[3], r[7], &tt, &b1, &b2, err, &cnt);
+    trace<false, true, SPH, L>(sc, rp, r[3], r[7], &tt, &b1, &b2, err, &cnt);
   }
   atomicAdd(&counters[0], (unsigned long long)cnt.nodes);
   atomicAdd(&counters[1], (unsigned long long)cnt.tris);
@@ -2189,6 +2642,15 @@ static void with_bool(bool b, F&& f) {
   else f(std::false_type{});
 }
 
+// Calls f with the active surface layout (a kLayout constant).
+template <class F>
+static void with_layout(const DevScene& s, F&& f) {
+  if (s.wide != 0) f(std::integral_constant<int, kLayout8>{});
+  else if (!s.nodes4) f(std::integral_constant<int, kLayout2>{});
+  else if (s.nodes4_bytes) f(std::integral_constant<int, kLayout4Bytes>{});
+  else f(std::integral_constant<int, kLayout4>{});
+}
+
 // Launch grids depend on the device's SM count, so they are cached per device ordinal
 // (the current device of the calling thread).  Concurrent first calls compute the same value.
 constexpr int kGridCacheDevices = 64;
@@ -2263,7 +2725,7 @@ void launch_extend(const DevScene& s, const PathState& p, int bounce, bool count
   const int b = blk(s);
   with_bool(count, [&](auto C) {
     with_bool(s.num_spheres > 0, [&](auto S) {
-      with_bool(s.wide != 0, [&](auto W) {
+      with_layout(s, [&](auto W) {
         auto* k = k_extend<decltype(C)::value, decltype(S)::value, decltype(W)::value>;
         k<<<full_grid(k, b), b, 0, st>>>(s, p, bounce, stats);
       });
@@ -2315,7 +2777,7 @@ void launch_shadow(const DevScene& s, const PathState& p, const Framebuffer& fb,
   with_bool(s.num_media > 0, [&](auto M) {
     with_bool(count, [&](auto C) {
       with_bool(s.num_spheres > 0, [&](auto S) {
-        with_bool(s.wide != 0, [&](auto W) {
+        with_layout(s, [&](auto W) {
           auto* k = k_shadow<decltype(M)::value, decltype(C)::value, decltype(S)::value, decltype(W)::value>;
           k<<<full_grid(k, b), b, 0, st>>>(s, p, fb, bounce, stats);
         });
@@ -2411,13 +2873,18 @@ static int grid_for(int n) {
   int g = (n + kBlock - 1) / kBlock;
   return g < 1 ? 1 : (g > 65535 ? 65535 : g);
 }
+// Blocks of a ray-batch launch: the device filled once, fewer for small batches.
+template <class K>
+static int batch_grid(K* kernel, int n) {
+  return std::min(full_grid(kernel, kBlock), grid_for(n));
+}
 void launch_intersect_rays(const DevScene& s, const float* rays, int n, int* prim, float* t, float* u, float* v,
                            unsigned int* err, cudaStream_t st) {
   if (n <= 0) return;
   with_bool(s.num_spheres > 0, [&](auto S) {
-    with_bool(s.wide != 0, [&](auto W) {
-      k_intersect_rays<decltype(S)::value, decltype(W)::value><<<grid_for(n), kBlock, 0, st>>>(s, rays, n, prim, t, u, v,
-                                                                                               err);
+    with_layout(s, [&](auto W) {
+      auto* k = k_intersect_rays<decltype(S)::value, decltype(W)::value>;
+      k<<<batch_grid(k, n), kBlock, 0, st>>>(s, rays, n, prim, t, u, v, err);
     });
   });
 }
@@ -2425,8 +2892,9 @@ void launch_occluded_rays(const DevScene& s, const float* rays, int n, unsigned 
                           cudaStream_t st) {
   if (n <= 0) return;
   with_bool(s.num_spheres > 0, [&](auto S) {
-    with_bool(s.wide != 0, [&](auto W) {
-      k_occluded_rays<decltype(S)::value, decltype(W)::value><<<grid_for(n), kBlock, 0, st>>>(s, rays, n, occ, err);
+    with_layout(s, [&](auto W) {
+      auto* k = k_occluded_rays<decltype(S)::value, decltype(W)::value>;
+      k<<<batch_grid(k, n), kBlock, 0, st>>>(s, rays, n, occ, err);
     });
   });
 }
@@ -2434,7 +2902,7 @@ void launch_count_rays(const DevScene& s, const float* rays, int n, unsigned lon
                        cudaStream_t st) {
   if (n <= 0) return;
   with_bool(s.num_spheres > 0, [&](auto S) {
-    with_bool(s.wide != 0, [&](auto W) {
+    with_layout(s, [&](auto W) {
       k_count_rays<decltype(S)::value, decltype(W)::value><<<grid_for(n), kBlock, 0, st>>>(s, rays, n, counters, err);
     });
   });
