@@ -4,6 +4,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <climits>
 #include <chrono>
 #include <cmath>
 #include <cstddef>
@@ -188,6 +189,51 @@ struct DeviceBuffers {
   }
 };
 
+// Page-locked areas that k_extend reports its queue lengths into, one per context that renders,
+// reused by later contexts (at most 16 kept).
+class CountAreas {
+ public:
+  static constexpr size_t kEntries = 1024;  // bounces: max_ray_depth <= 1000
+  static unsigned long long* take() {
+    {
+      std::lock_guard<std::mutex> g(mu());
+      if (!kept().empty()) {
+        unsigned long long* p = kept().back();
+        kept().pop_back();
+        return p;
+      }
+    }
+    void* p = nullptr;
+    if (cudaHostAlloc(&p, kEntries * sizeof(unsigned long long), cudaHostAllocPortable | cudaHostAllocMapped) !=
+        cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
+    return static_cast<unsigned long long*>(p);
+  }
+  static void give(unsigned long long* p) {
+    if (!p) return;
+    {
+      std::lock_guard<std::mutex> g(mu());
+      if (kept().size() < 16) {
+        kept().push_back(p);
+        return;
+      }
+    }
+    cudaFreeHost(p);
+  }
+
+ private:
+  static std::mutex& mu() {
+    static std::mutex* m = new std::mutex;
+    return *m;
+  }
+  static std::vector<unsigned long long*>& kept() {
+    static auto* v = new std::vector<unsigned long long*>;
+    return *v;
+  }
+};
+
 std::mutex g_pool_mutex;
 cudaMemPool_t g_pools[64] = {nullptr};
 
@@ -281,6 +327,8 @@ struct tt_ctx {
   unsigned int* d_err = nullptr;
   int grid = 0;
   int wave_cap = 0;
+  unsigned long long* host_counts = nullptr;  // queue lengths of the running wave (CountAreas)
+  unsigned wave_tag = 0;
   int rounds = 0;
   // Accumulation bookkeeping.
   std::vector<uint64_t> spp_count;
@@ -1419,6 +1467,38 @@ static tt_status guide_train(tt_ctx* c, long long paths) {
   return TT_OK;
 }
 
+// A wave runs as whole paths in one launch from its camera samples up to kWholePaths, and from
+// the bounce on where at most kTailPaths are left.  k_paths serves few paths at the latency of one
+// path's stages; with many it is 2-4 times slower than the wavefront kernels (96-128 registers with
+// spills, every lane in its own material).  64x64 pixels, k_paths against the wavefront: Cornell
+// box 0.17 / 0.49 ms at 1 sample, 0.50 / 0.65 at 32 (131,072 paths); with medium 0.53 / 1.72 and
+// 2.28 / 2.47; terrain 0.34 / 1.26 and 1.93 / 2.75.  Tail limits of 4,096 / 32,768 / 65,536 /
+// 262,144 paths: terrain 641x359 x 1 2.23 / 1.81 / 1.75 / 1.95 ms (3.25 without), medium box
+// 512x512 x 8 8.11 / 8.06 / 8.09 / 8.27 (8.39), planet 7.12 / 6.97 / 6.99 / 7.06 (8.48).
+constexpr int kWholePaths = 1 << 17;
+constexpr int kTailPaths = 1 << 16;
+
+// Starts a new wave's queue-length reports.
+static void next_wave_tag(tt_ctx* c) {
+  if (!c->host_counts) c->host_counts = CountAreas::take();
+  c->ps.host_counts = c->host_counts;
+  c->ps.wave_tag = ++c->wave_tag;
+}
+
+// Length of bounce b's extension queue as its k_extend reported it; waits for that launch to
+// start.  Large when the stream ended without a report (an error, found by the caller later).
+static unsigned reported_count(tt_ctx* c, int b) {
+  const volatile unsigned long long* v = c->host_counts + b;
+  for (unsigned spin = 1;; ++spin) {
+    const unsigned long long x = *v;
+    if ((unsigned)(x >> 32) == c->wave_tag) return (unsigned)x;
+    if ((spin & 0xfffu) == 0u && cudaStreamQuery(c->stream) != cudaErrorNotReady) {
+      const unsigned long long y = *v;
+      return (unsigned)(y >> 32) == c->wave_tag ? (unsigned)y : 0xffffffffu;
+    }
+  }
+}
+
 static tt_status render_range(tt_ctx* c, int32_t spp, uint64_t seed, int32_t pb, int32_t pe) {
   if (!c) return TT_ERR_INVALID;
   if (!c->uploaded) return fail(c, TT_ERR_NOT_READY, "tt_upload_scene has not run");
@@ -1461,7 +1541,7 @@ static tt_status render_range(tt_ctx* c, int32_t spp, uint64_t seed, int32_t pb,
   TT_CUDA(c, cudaEventRecord(pass_begin, c->stream));
   const int grid = c->grid;
   const int rounds = c->rounds;
-  uint64_t launches = 0;
+  uint64_t launches = 0, extend_launches = 0, shadow_launches = 0;
   bool stopped = false;
   int wave_index = 0;
   for (long long ws = 0; ws < total; ws += cap, ++wave_index) {
@@ -1476,28 +1556,51 @@ static tt_status render_range(tt_ctx* c, int32_t spp, uint64_t seed, int32_t pb,
     w.sample_offset = c->next_sample;
     w.seed = seed;
     cudaMemsetAsync(c->ps.counters, 0, kCountersPerBounce * (size_t)(rounds + 3) * sizeof(int), c->stream);
-    launch_generate(c->dev, c->ps, c->fb, w, grid, c->stream);
-    launches++;
-    for (int b = 0; b < rounds; ++b) {
-      timed(1, [&] { launch_shadow(c->dev, c->ps, c->fb, b, counting, c->d_stats + 2, grid, c->stream); });
-      if (c->dev.guide_record) launch_flush(c->dev, c->ps, c->fb, b, grid, c->stream);
-      timed(0, [&] { launch_extend(c->dev, c->ps, b, counting, c->d_stats, grid, c->stream); });
-      if (c->dev.num_media > 0) {
-        launch_track(c->dev, c->ps, b, grid, c->stream);
-        launches++;
+    // Small waves run as whole paths in one launch; larger ones bounce by bounce, the last
+    // bounces' few paths as whole paths again (after the guided bounces).  Not with guiding
+    // records, nor when single launches are timed or counted.
+    const bool whole = !c->dev.guide_record && !timing && c->dev.algo == TT_ALGO_PT && !c->dev.wide;
+    const bool fused = whole && !c->dev.guide && w.wave_paths <= kWholePaths &&
+                       launch_paths(c->dev, c->ps, c->fb, w, -1, rounds, INT_MAX, kFlushNone, c->d_stats, c->stream);
+    if (!fused) {
+      if (whole) next_wave_tag(c);
+      else c->ps.host_counts = nullptr;
+      launch_generate(c->dev, c->ps, c->fb, w, grid, c->stream);
+      launches++;
+      const int tail = std::max(2, c->dev.guide ? c->dev.guide_depth : 0);
+      int b = 0;
+      for (; b < rounds; ++b) {
+        timed(1, [&] { launch_shadow(c->dev, c->ps, c->fb, b, counting, c->d_stats + 2, grid, c->stream); });
+        ++shadow_launches;
+        if (c->dev.guide_record) launch_flush(c->dev, c->ps, c->fb, b, grid, c->stream);
+        // The launches of bounce b - 1 keep the device busy while the host reads its count.
+        if (c->ps.host_counts && b >= tail && reported_count(c, b - 1) <= (unsigned)kTailPaths &&
+            launch_paths(c->dev, c->ps, c->fb, w, b, rounds, INT_MAX, kFlushNone, c->d_stats, c->stream)) {
+          launches += 2;
+          break;
+        }
+        timed(0, [&] { launch_extend(c->dev, c->ps, b, counting, c->d_stats, grid, c->stream); });
+        ++extend_launches;
+        if (c->dev.num_media > 0) {
+          launch_track(c->dev, c->ps, b, grid, c->stream);
+          launches++;
+        }
+        launch_shade(c->dev, c->ps, b, grid, c->stream);
+        if (c->dev.guide && b < c->dev.guide_depth) {
+          launch_guide(c->dev, c->ps, b, c->stream);
+          launches++;
+        }
+        launches += (c->dev.guide_record ? 3 : 2) + shade_launches(c->dev, c->ps, b);
       }
-      launch_shade(c->dev, c->ps, b, grid, c->stream);
-      if (c->dev.guide && b < c->dev.guide_depth) {
-        launch_guide(c->dev, c->ps, b, c->stream);
-        launches++;
+      if (b == rounds) {
+        timed(1, [&] { launch_shadow(c->dev, c->ps, c->fb, rounds, counting, c->d_stats + 2, grid, c->stream); });
+        ++shadow_launches;
       }
-      launches += (c->dev.guide_record ? 3 : 2) + shade_launches(c->dev, c->ps, b);
     }
-    timed(1, [&] { launch_shadow(c->dev, c->ps, c->fb, rounds, counting, c->d_stats + 2, grid, c->stream); });
     // Finished paths into the pass framebuffer: with guiding records, k_flush after every
     // bounce (it also commits the records); without, one gather at the end of the wave.
     if (c->dev.guide_record) launch_flush(c->dev, c->ps, c->fb, rounds, grid, c->stream);
-    else launch_gather(c->dev, c->ps, c->fb, w, grid, c->stream);
+    else launch_gather(c->ps, c->fb, w, fused, grid, c->stream);
     k_tally<<<1, 32, 0, c->stream>>>(c->ps.counters, rounds, c->d_stats);
     launches += 3;
     cudaEventRecord(wave_ev[wave_index & 1], c->stream);
@@ -1519,8 +1622,8 @@ static tt_status render_range(tt_ctx* c, int32_t spp, uint64_t seed, int32_t pb,
     cudaEventDestroy(ev[2 * k + 1]);
   }
   if (!timing) {
-    c->stats.extend_launches += (uint64_t)rounds * wave_index;
-    c->stats.shadow_launches += (uint64_t)(rounds + 1) * wave_index;
+    c->stats.extend_launches += extend_launches;
+    c->stats.shadow_launches += shadow_launches;
   }
   cudaEventDestroy(pass_begin);
   cudaEventDestroy(pass_end);
@@ -1932,6 +2035,7 @@ void tt_destroy(tt_ctx* c) {
   if (c->stream) cudaStreamSynchronize(c->stream);
   if (c->d_records) cudaFree(c->d_records);
   if (c->d_rec_count) cudaFree(c->d_rec_count);
+  CountAreas::give(c->host_counts);
   c->gnet.reset();
   c->tree.reset();
   c->path_mem.free_all();
@@ -2407,24 +2511,48 @@ static tt_status render_views(tt_ctx* c, const tt_view* views, int32_t n, uint64
   const int rounds = c->rounds;
   const DevScene& sc = c->dev;
   PathState& ps = c->ps;
-  auto wave = [&](cudaStream_t s) {
+  // One wave's launches.  eager: the host watches the queue lengths and ends the wave with whole
+  // paths; in a captured wave the same launch sits behind several bounces and takes over where its
+  // own limit is met.  Returns the kernels launched.
+  WaveArgs none{};
+  auto wave = [&](cudaStream_t s, bool eager) {
+    int k = 2;
+    const bool whole = !sc.guide_record && sc.algo == TT_ALGO_PT && !sc.wide;
+    const int tail = std::max(2, sc.guide ? sc.guide_depth : 0);
+    if (eager && whole) next_wave_tag(c);
+    else ps.host_counts = nullptr;
     cudaMemsetAsync(ps.counters, 0, kCountersPerBounce * (size_t)(rounds + 3) * sizeof(int), s);
     launch_generate_views(sc, ps, d_waves, d_idx, d_views, n, grid, s);
-    for (int b = 0; b < rounds; ++b) {
+    int b = 0;
+    for (; b < rounds; ++b) {
       launch_shadow(sc, ps, fb, b, false, nullptr, grid, s);
       launch_flush(sc, ps, fb, b, grid, s);
+      k += 2;
+      if (eager) {
+        if (ps.host_counts && b >= tail && reported_count(c, b - 1) <= (unsigned)kTailPaths &&
+            launch_paths(sc, ps, fb, none, b, rounds, INT_MAX, kFlushNow, c->d_stats, s)) {
+          ++k;
+          break;
+        }
+      } else if (whole && b >= tail && b % 4 == 0 &&
+                 launch_paths(sc, ps, fb, none, b, rounds, kTailPaths, kFlushCaptured, c->d_stats, s)) {
+        k += 2;
+      }
       launch_extend(sc, ps, b, false, nullptr, grid, s);
       if (sc.num_media > 0) launch_track(sc, ps, b, grid, s);
       launch_shade(sc, ps, b, grid, s);
       if (sc.guide && b < sc.guide_depth) launch_guide(sc, ps, b, s);
+      k += 1 + (sc.num_media > 0) + shade_launches(sc, ps, b) + (sc.guide && b < sc.guide_depth);
     }
-    launch_shadow(sc, ps, fb, rounds, false, nullptr, grid, s);
-    launch_flush(sc, ps, fb, rounds, grid, s);
+    if (b == rounds) {
+      launch_shadow(sc, ps, fb, rounds, false, nullptr, grid, s);
+      launch_flush(sc, ps, fb, rounds, grid, s);
+      k += 2;
+    }
     k_tally<<<1, 32, 0, s>>>(ps.counters, rounds, c->d_stats);
     launch_wave_advance(d_idx, s);
+    return k + 1;
   };
-  int per_wave = 4 + rounds * (3 + (sc.num_media > 0)) + (sc.guide ? std::min(rounds, sc.guide_depth) : 0) + 2;
-  for (int b = 0; b < rounds; ++b) per_wave += shade_launches(sc, ps, b);
   cudaEventCreate(&ev0);
   cudaEventCreate(&ev1);
   cudaEventRecord(ev0, c->stream);
@@ -2432,13 +2560,13 @@ static tt_status render_views(tt_ctx* c, const tt_view* views, int32_t n, uint64
   int done_waves = 0;
   for (cudaEvent_t& e : wave_end)
     if ((st = check(cudaEventCreate(&e))) != TT_OK) return st;
-  wave(c->stream);  // eager first wave
+  uint64_t launches = (uint64_t)wave(c->stream, true);  // eager first wave
   cudaEventRecord(wave_end[0], c->stream);
   ++done_waves;
   if ((st = check(cudaGetLastError())) != TT_OK) return st;
   if (nwaves > 1) {
     if ((st = check(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal))) != TT_OK) return st;
-    wave(c->stream);
+    const int per_wave = wave(c->stream, false);
     cudaError_t ce = cudaStreamEndCapture(c->stream, &graph);
     if (ce == cudaSuccess) ce = cudaGraphInstantiate(&exec, graph, 0);
     if ((st = check(ce)) != TT_OK) return st;
@@ -2446,6 +2574,7 @@ static tt_status render_views(tt_ctx* c, const tt_view* views, int32_t n, uint64
       if (c->stop.load()) { stopped = true; break; }
       if ((st = check(cudaGraphLaunch(exec, c->stream))) != TT_OK) return st;
       cudaEventRecord(wave_end[done_waves], c->stream);
+      launches += (uint64_t)per_wave;
     }
   }
   launch_resolve_views(d_acc, d_light, d_views, n, (int)npix_total, d_rgb, c->stream);
@@ -2466,7 +2595,7 @@ static tt_status render_views(tt_ctx* c, const tt_view* views, int32_t n, uint64
     if (w < done_waves) cudaEventElapsedTime(&c->views_done_ms[v], ev0, wave_end[w]);
   }
   c->stats.pass_ms += ms;
-  c->stats.kernel_launches += (uint64_t)done_waves * per_wave + 1;
+  c->stats.kernel_launches += launches + 1;
   c->stats.extend_launches += (uint64_t)done_waves * rounds;
   c->stats.shadow_launches += (uint64_t)done_waves * (rounds + 1);
   c->stats.paths += (uint64_t)std::min<long long>(paths, (long long)done_waves * cap);

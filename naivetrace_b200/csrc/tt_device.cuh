@@ -195,8 +195,10 @@ __device__ __forceinline__ float3 to_triangle_barycentric(const float r[2]) {
   return f3(1.f - s, (1.f - r[1]) * s, r[1] * s);
 }
 __device__ __forceinline__ float power_heuristic(float p, float o) {
-  float pp = p * p;
-  return pp / (pp + o * o + kEps);
+  // The rounding is fixed: whether a compiler contracts p * p or o * o would differ between the
+  // kernels that share this.
+  const float pp = __fmul_rn(p, p);
+  return pp / __fadd_rn(__fmaf_rn(o, o, pp), kEps);
 }
 __device__ __forceinline__ int tower_sampling4(const float* probs, float r) {
   int n = 3;

@@ -197,6 +197,10 @@ struct PathState {
   int* sort_q;         // material-sorted hit queue (sort_shading only, else null)
   unsigned char* sort_key;  // shading key per entry of the bounce's hit queue
   unsigned int* err;
+  // Extension-queue length of each bounce, written by k_extend into page-locked host memory as
+  // wave_tag << 32 | length, so that the host sees how many paths are left (null: not wanted).
+  unsigned long long* host_counts;
+  unsigned wave_tag;
   // Media scenes only (null otherwise).
   uint2* track;        // medium tracker: x = 4 slot bytes (0xff empty), y = current medium (-1 vacuum)
   float4* vol;         // sigma_s at a volume interaction (xyz); w = transmittance pdf factor of the step
@@ -279,9 +283,19 @@ void launch_flush(const DevScene& s, const PathState& p, const Framebuffer& fb, 
                   cudaStream_t st);
 // End of a wave without guiding records: every path's accumulator is final, so each pixel
 // of the pass range sums the RGB of its paths in the wave (its slots npix_range apart, in
-// sample order) into the pass framebuffer; this replaces the wave's k_flush launches.
-void launch_gather(const DevScene& s, const PathState& p, const Framebuffer& fb, const WaveArgs& w, int grid,
-                   cudaStream_t st);
+// sample order) into the pass framebuffer; this replaces the wave's k_flush launches.  rgb: the
+// paths were finished by launch_paths from their camera samples, whose accumulators hold RGB.
+void launch_gather(const PathState& p, const Framebuffer& fb, const WaveArgs& w, bool rgb, int grid, cudaStream_t st);
+// Whole paths in one launch (algo pt, binary or 4-wide layout; without guided vertices or guiding
+// records): first < 0 the wave's camera samples, else the paths of bounce `first`'s extension
+// queue, whose shadow rays of that bounce have been traced; nothing when there are more than
+// max_n.  Finished paths stay in accum for the gather, or go straight into the framebuffer
+// (kFlushNow; kFlushCaptured for waves whose later launches are queued already: it empties the
+// queue it took and counts rays in stats[4] and stats[5] instead of the bounces' queue lengths).
+// Returns false, launching nothing, for other variants.
+enum { kFlushNone = 0, kFlushNow = 1, kFlushCaptured = 2 };
+bool launch_paths(const DevScene& s, const PathState& p, const Framebuffer& fb, const WaveArgs& w, int first, int rounds,
+                  int max_n, int flush, unsigned long long* stats, cudaStream_t st);
 // Guided scenes: network evaluation and one-sample MIS scattering of the queued guided
 // vertices (persistent kernel, as many CTAs as fit on the SMs).
 void launch_guide(const DevScene& s, const PathState& p, int bounce, cudaStream_t st);
