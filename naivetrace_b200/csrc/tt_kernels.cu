@@ -980,6 +980,7 @@ __device__ __forceinline__ void trace8_run(const uint4* __restrict__ nodes, cons
 template <bool ANY, bool COUNT, bool SPH, int L>
 __device__ __forceinline__ int trace(const DevScene& sc, const RayPre& r, float tnear, float tfar, float* t_out,
                                      float* b1_out, float* b2_out, unsigned int* err, TraceCounters* cnt) {
+  static_assert(L == kLayout2 || L == kLayout4 || L == kLayout4Bytes || L == kLayout8, "not a layout");
   if constexpr (L == kLayout8) {
     Trace8State s;
     s.tnear = tnear;
@@ -3141,7 +3142,7 @@ void launch_shadow(const DevScene& s, const PathState& p, const Framebuffer& fb,
   const int b = blk(s);
   if (s.algo == TT_ALGO_PT2 && s.num_media > 0) {
     with_bool(s.num_spheres > 0, [&](auto S) {
-      with_bool(s.wide != 0, [&](auto W) {
+      with_layout(s, [&](auto W) {
         auto* k = k_shadow2<decltype(S)::value, decltype(W)::value>;
         k<<<full_grid(k, b), b, 0, st>>>(s, p, bounce);
       });

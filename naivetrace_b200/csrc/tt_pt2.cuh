@@ -470,8 +470,9 @@ __global__ void __launch_bounds__(256) k_shade2(DevScene sc, PathState p, int bo
 // transmission through the medium segments on the shadow ray's own stream, then the MIS
 // weight over the hero wavelengths (the end of AddDirectLighting, :537-560).  Without media
 // the contribution is final at the vertex and the plain shadow kernel adds it.
-template <bool SPH, bool WIDE>
+template <bool SPH, int L>
 __global__ void __launch_bounds__(256) k_shadow2(DevScene sc, PathState p, int bounce) {
+  constexpr bool WIDE = L == kLayout8;
   const int n = *sh_count(p, bounce);
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const int slot = p.sh_q[i];
@@ -479,7 +480,7 @@ __global__ void __launch_bounds__(256) k_shadow2(DevScene sc, PathState p, int b
     const RayPre r = prepare_ray(xyz(o), xyz(d));
     float t, b1, b2;
     TraceCounters cnt{0u, 0u};
-    const int hit = trace<true, false, SPH, WIDE>(sc, r, 0.f, o.w, &t, &b1, &b2, p.err, &cnt);
+    const int hit = trace<true, false, SPH, L>(sc, r, 0.f, o.w, &t, &b1, &b2, p.err, &cnt);
     if (hit >= 0) continue;
     const Lambda l = unpack_lambda(p.meta[slot].y);
     MTracker mt = load_tracker(p.sh_track[slot]);

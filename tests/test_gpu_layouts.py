@@ -3,7 +3,7 @@ with float boxes, bit for bit, around the primitive count where the format chang
 import numpy as np
 import pytest
 
-from naivetrace_b200 import scenes
+from naivetrace_b200 import abi, scenes
 from naivetrace_b200.algo import GpuContext
 from naivetrace_b200.scene import Scene, diffuse, make_params
 
@@ -62,3 +62,21 @@ def test_byte_boxes_equal_binary(prims, spheres, offset, monkeypatch):
             assert np.array_equal(a, b)
         assert np.array_equal(wide.occluded(rays), binary.occluded(rays))
     assert wide.stats()["error_flags"] == 0
+
+
+@pytest.mark.parametrize("algo", [abi.ALGO_PT, abi.ALGO_PT2])
+@pytest.mark.parametrize("name", ["cornell_box_media_mix", "spheres_box"])
+def test_renders_on_every_layout(algo, name, monkeypatch):
+    """Media renders on the binary and the 8-wide layout: every kernel traverses the layout the
+    context holds."""
+    params = make_params(max_ray_depth=8, algo=algo)
+    images = []
+    for width in ("4", "2", "8"):
+        monkeypatch.setenv("TT_BVH_WIDTH", width)
+        g = GpuContext(getattr(scenes, name)(48, 40), params)
+        g.render(4, seed=2)
+        images.append(g.accumulators()[0])
+        assert g.stats()["error_flags"] == 0
+    assert np.array_equal(images[0], images[1])
+    # The 8-wide layout's own boxes may decide a grazing ray otherwise.
+    assert np.isclose(images[0], images[2], rtol=1e-5, atol=1e-6).mean() > 0.999
