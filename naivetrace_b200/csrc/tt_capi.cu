@@ -1789,7 +1789,7 @@ tt_status tt_intersect_batch(tt_ctx* c, const float* rays, int32_t n, int32_t* p
   cudaMalloc(&du, n * sizeof(float));
   cudaMalloc(&dv, n * sizeof(float));
   cudaMalloc(&dp, n * sizeof(int));
-  cudaMemcpy(dr, rays, 8 * (size_t)n * sizeof(float), cudaMemcpyHostToDevice);
+  cudaMemcpyAsync(dr, rays, 8 * (size_t)n * sizeof(float), cudaMemcpyHostToDevice, c->stream);
   launch_intersect_rays(c->dev, dr, n, dp, dt, du, dv, c->d_err, c->stream);
   cudaStreamSynchronize(c->stream);
   cudaError_t e = cudaGetLastError();
@@ -1809,7 +1809,7 @@ tt_status tt_occluded_batch(tt_ctx* c, const float* rays, int32_t n, uint8_t* oc
   unsigned char* docc = nullptr;
   TT_CUDA(c, cudaMalloc(&dr, 8 * (size_t)n * sizeof(float)));
   TT_CUDA(c, cudaMalloc(&docc, n));
-  cudaMemcpy(dr, rays, 8 * (size_t)n * sizeof(float), cudaMemcpyHostToDevice);
+  cudaMemcpyAsync(dr, rays, 8 * (size_t)n * sizeof(float), cudaMemcpyHostToDevice, c->stream);
   launch_occluded_rays(c->dev, dr, n, docc, c->d_err, c->stream);
   cudaStreamSynchronize(c->stream);
   cudaError_t e = cudaGetLastError();
@@ -1835,7 +1835,7 @@ tt_status tt_count_traversal(tt_ctx* c, const float* rays, int32_t n) {
   if (st != TT_OK || n == 0) return st;
   float* dr = nullptr;
   TT_CUDA(c, cudaMalloc(&dr, 8 * (size_t)n * sizeof(float)));
-  cudaMemcpy(dr, rays, 8 * (size_t)n * sizeof(float), cudaMemcpyHostToDevice);
+  cudaMemcpyAsync(dr, rays, 8 * (size_t)n * sizeof(float), cudaMemcpyHostToDevice, c->stream);
   launch_count_rays(c->dev, dr, n, c->d_stats, c->d_err, c->stream);
   cudaStreamSynchronize(c->stream);
   cudaError_t e = cudaGetLastError();
@@ -1884,7 +1884,7 @@ tt_status tt_eval_bsdf_batch(tt_ctx* c, int32_t material, const float* wi, const
   TT_CUDA(c, cudaMalloc(&di, 3 * (size_t)n * sizeof(float)));
   TT_CUDA(c, cudaMalloc(&dv, 3 * (size_t)n * sizeof(float)));
   TT_CUDA(c, cudaMalloc(&dp, (size_t)n * sizeof(float)));
-  cudaMemcpy(di, dirs, 3 * (size_t)n * sizeof(float), cudaMemcpyHostToDevice);
+  cudaMemcpyAsync(di, dirs, 3 * (size_t)n * sizeof(float), cudaMemcpyHostToDevice, c->stream);
   launch_eval_bsdf(c->dev, material, make_float3(wi[0], wi[1], wi[2]), make_int3(li[0], li[1], li[2]), di, n, dv, dp,
                    c->stream);
   cudaStreamSynchronize(c->stream);
@@ -1936,7 +1936,7 @@ tt_status tt_eval_phase_batch(tt_ctx* c, int32_t medium, const float* pos, const
   TT_CUDA(c, cudaMalloc(&di, 3 * (size_t)n * sizeof(float)));
   TT_CUDA(c, cudaMalloc(&dv, 3 * (size_t)n * sizeof(float)));
   TT_CUDA(c, cudaMalloc(&dp, (size_t)n * sizeof(float)));
-  cudaMemcpy(di, dirs, 3 * (size_t)n * sizeof(float), cudaMemcpyHostToDevice);
+  cudaMemcpyAsync(di, dirs, 3 * (size_t)n * sizeof(float), cudaMemcpyHostToDevice, c->stream);
   launch_eval_phase(c->dev, medium, make_float3(pos[0], pos[1], pos[2]), make_float3(wi[0], wi[1], wi[2]),
                     make_int3(li[0], li[1], li[2]), di, n, dv, dp, c->stream);
   cudaStreamSynchronize(c->stream);
@@ -2160,7 +2160,7 @@ static tt_status guide_forward(tt_ctx* c, const float* features, int32_t n, floa
   if (!c->gnet->ensure_capacity(n, &gerr)) return fail(c, TT_ERR_CUDA, gerr);
   std::vector<__nv_bfloat16> x((size_t)n * kGIn);
   for (size_t i = 0; i < x.size(); ++i) x[i] = __float2bfloat16(features[i]);
-  TT_CUDA(c, cudaMemcpy(c->gnet->x0, x.data(), x.size() * sizeof(__nv_bfloat16), cudaMemcpyHostToDevice));
+  TT_CUDA(c, cudaMemcpyAsync(c->gnet->x0, x.data(), x.size() * sizeof(__nv_bfloat16), cudaMemcpyHostToDevice, c->stream));
   if (tcgen05) {
     if (!c->gnet->forward_tc(c->gnet->x0, n, c->gnet->out, c->stream))
       return fail(c, TT_ERR_LOOP_CAP, "tensor-core forward: a wait timed out");
@@ -2189,7 +2189,7 @@ static tt_status guide_batch(tt_ctx* c, const float* records, int32_t n, int32_t
   if (!c->gnet->ensure_capacity(n, &gerr)) return fail(c, TT_ERR_CUDA, gerr);
   GuideRecord* d = nullptr;
   TT_CUDA(c, cudaMalloc(&d, (size_t)n * sizeof(GuideRecord)));
-  cudaError_t e = cudaMemcpy(d, records, (size_t)n * sizeof(GuideRecord), cudaMemcpyHostToDevice);
+  cudaError_t e = cudaMemcpyAsync(d, records, (size_t)n * sizeof(GuideRecord), cudaMemcpyHostToDevice, c->stream);
   for (int k = 0; k < steps && e == cudaSuccess; ++k) {
     c->gnet->gradient(d, n, c->stream, train, lr);
   }
@@ -2220,7 +2220,7 @@ tt_status tt_guide_gradient_pool_batch(tt_ctx* c, const float* pool, int32_t poo
   if (!c->gnet->ensure_capacity(n, &gerr)) return fail(c, TT_ERR_CUDA, gerr);
   GuideRecord* d = nullptr;
   TT_CUDA(c, cudaMalloc(&d, (size_t)pool_n * sizeof(GuideRecord)));
-  cudaError_t e = cudaMemcpy(d, pool, (size_t)pool_n * sizeof(GuideRecord), cudaMemcpyHostToDevice);
+  cudaError_t e = cudaMemcpyAsync(d, pool, (size_t)pool_n * sizeof(GuideRecord), cudaMemcpyHostToDevice, c->stream);
   if (e == cudaSuccess) {
     c->gnet->gradient(d, n, c->stream, false, 0.f, pool_n, seed);
     e = cudaStreamSynchronize(c->stream);
@@ -2400,7 +2400,7 @@ tt_status tt_guide_features_batch(tt_ctx* c, const float* points, int32_t n, flo
     cudaFree(dp);
     return fail(c, TT_ERR_CUDA, "allocation failed");
   }
-  cudaError_t e = cudaMemcpy(dp, points, (size_t)n * 9 * sizeof(float), cudaMemcpyHostToDevice);
+  cudaError_t e = cudaMemcpyAsync(dp, points, (size_t)n * 9 * sizeof(float), cudaMemcpyHostToDevice, c->stream);
   if (e == cudaSuccess) {
     c->gnet->features(dp, n, dx, c->stream);
     e = cudaStreamSynchronize(c->stream);
