@@ -39,14 +39,6 @@ __device__ __forceinline__ void m33_acc(M33f& w, const M33f& x) {
 #pragma unroll
   for (int k = 0; k < 9; ++k) w.a[k] = fix_nan(w.a[k] * x.a[k]);
 }
-// AccumulateContributions(w, f, p) (:231-238): w_ij *= p_j / f_i.
-__device__ __forceinline__ void m33_acc(M33f& w, float3 f, float3 p) {
-  const float fi[3] = {f.x, f.y, f.z}, pj[3] = {p.x, p.y, p.z};
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int j = 0; j < 3; ++j) w.a[3 * i + j] = fix_nan(w.a[3 * i + j] * fix_nan((1.f / fi[i]) * pj[j]));
-}
 __device__ __forceinline__ float3 m33_row_mean(const M33f& m) {
   return f3((m.a[0] + m.a[1] + m.a[2]) * (1.f / 3.f), (m.a[3] + m.a[4] + m.a[5]) * (1.f / 3.f),
             (m.a[6] + m.a[7] + m.a[8]) * (1.f / 3.f));
@@ -88,8 +80,24 @@ __device__ __forceinline__ float3 exp_maj(float3 maj, float x) {
   return f3(expf(-x * maj.x), expf(-x * maj.y), expf(-x * maj.z));
 }
 
+// AccumulateContributions(w, f, p) (media_integrator.cxx:231-238) for two matrices with the same f: wa_ij *= f_j / f_i and
+// wb_ij *= p_j / f_i.
+__device__ __forceinline__ void m33_acc2(M33f& wa, M33f& wb, float3 f, float3 p) {
+  const float inv[3] = {1.f / f.x, 1.f / f.y, 1.f / f.z}, fj[3] = {f.x, f.y, f.z}, pj[3] = {p.x, p.y, p.z};
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      wa.a[3 * i + j] = fix_nan(wa.a[3 * i + j] * fix_nan(inv[i] * fj[j]));
+      wb.a[3 * i + j] = fix_nan(wb.a[3 * i + j] * fix_nan(inv[i] * pj[j]));
+    }
+}
+
 // nullpath::Tracking on one segment: hero-wavelength delta tracking.  Returns true at a
 // real collision, at distance *t_out.  At most 10^4 steps (then no collision).
+// The three ends of a step choose factors and share one accumulation: k_shade2 was bound by
+// instruction fetch (11 of 18 cycles per issue), and with an accumulation per end and matrix this
+// loop alone held six copies of it (pt2 in mixed media 320x240 x 8: 10.3 -> 9.6 ms).
 template <class R>
 __device__ __forceinline__ bool track_segment2(const DevScene& sc, int medium, float3 org, float3 dir, float len,
                                                M33f& ft, M33f& fn, R& rng, Lambda l, float* t_out) {
@@ -100,24 +108,25 @@ __device__ __forceinline__ bool track_segment2(const DevScene& sc, int medium, f
     const float tlocal = fminf(kLargeNumber, -logf(1.f - rng.uniform()) * mfp);
     const float3 tr = exp_maj(maj, fminf(tlocal, len - t));
     t += tlocal;
-    if (t >= len) {
-      m33_acc(ft, tr, tr);
-      m33_acc(fn, tr, tr);
-      return false;
+    float3 f = tr, pn = tr;
+    bool collided = false;
+    const bool end = t >= len;
+    if (!end) {
+      float3 ss, st;
+      coeffs2(sc, medium, org + dir * t, l, &ss, &st);
+      const float3 sn = maj - st;
+      const float prob_n = sn.x * mfp;
+      if (rng.uniform() < prob_n) {
+        f = mul(tr, sn);
+        pn = mul(tr, maj);
+      } else {
+        f = mul(tr, st);
+        collided = true;
+      }
     }
-    float3 ss, st;
-    coeffs2(sc, medium, org + dir * t, l, &ss, &st);
-    const float3 sn = maj - st;
-    const float prob_n = sn.x * mfp;
-    if (rng.uniform() < prob_n) {
-      m33_acc(ft, mul(tr, sn), mul(tr, sn));
-      m33_acc(fn, mul(tr, sn), mul(tr, maj));
-    } else {
-      m33_acc(ft, mul(tr, st), mul(tr, st));
-      m33_acc(fn, mul(tr, st), tr);
-      *t_out = t;
-      return true;
-    }
+    m33_acc2(ft, fn, f, pn);
+    if (collided) *t_out = t;
+    if (end || collided) return collided;
   }
   return false;
 }
@@ -137,16 +146,16 @@ __device__ __forceinline__ void transmit_segment2(const DevScene& sc, int medium
     const float tlocal = fminf(kLargeNumber, -logf(1.f - rng.uniform()) * mfp);
     const float3 tr = exp_maj(maj, fminf(tlocal, len - t));
     t += tlocal;
-    if (t >= len) {
-      m33_acc(st_, tr, tr);
-      m33_acc(sn_, tr, tr);
-      break;
+    float3 f = tr, pn = tr;
+    const bool end = t >= len;
+    if (!end) {
+      float3 ss, st;
+      coeffs2(sc, medium, org + dir * t, l, &ss, &st);
+      f = mul(tr, maj - st);
+      pn = mul(tr, maj);
     }
-    float3 ss, st;
-    coeffs2(sc, medium, org + dir * t, l, &ss, &st);
-    const float3 sn = maj - st;
-    m33_acc(st_, mul(tr, sn), mul(tr, sn));
-    m33_acc(sn_, mul(tr, sn), mul(tr, maj));
+    m33_acc2(st_, sn_, f, pn);
+    if (end) break;
     if (sn_.a[0] > kLargeNumber && sn_.a[4] > kLargeNumber && sn_.a[8] > kLargeNumber) {
 #pragma unroll
       for (int k = 0; k < 9; ++k) sn_.a[k] = INFINITY;
@@ -406,10 +415,9 @@ __global__ void __launch_bounds__(256) k_shade2(DevScene sc, PathState p, int bo
         }
         acc = acc + mis2<MEDIA>(sc, mul(rad, beta), has_last, last_pdf, last_delta, other, wt, wtn);
       }
-      if (sc.sample_lights) nee2<MEDIA>(sc, p, bounce + 1, slot, rng, l, beta, wi, &s, rough, -1, vpos, mt, wt);
-    } else if (!done) {
-      if (sc.sample_lights) nee2<MEDIA>(sc, p, bounce + 1, slot, rng, l, beta, wi, nullptr, rough, vmed, vpos, mt, wt);
     }
+    if (!done && sc.sample_lights)
+      nee2<MEDIA>(sc, p, bounce + 1, slot, rng, l, beta, wi, volume ? nullptr : &s, rough, vmed, vpos, mt, wt);
     const int count = count0 + 1;
     if (!done && count > sc.max_path_nodes - 1) done = true;
     rng.prep((unsigned)count0 << 1);
