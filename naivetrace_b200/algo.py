@@ -66,7 +66,7 @@ class GpuContext:
         self._check(self.render_pass(spp, seed, pixel_begin, pixel_end), "tt_render_pass")
 
     def framebuffer(self) -> np.ndarray:
-        rgb = np.zeros(3 * self.npix, np.float32)
+        rgb = np.empty(3 * self.npix, np.float32)
         self._check(self.lib.tt_read_framebuffer(self.h, _fp(rgb), None), "tt_read_framebuffer")
         return rgb
 
@@ -93,20 +93,20 @@ class GpuContext:
     def intersect(self, rays: np.ndarray):
         rays = np.ascontiguousarray(rays, dtype=np.float32).reshape(-1, 8)
         n = len(rays)
-        prim = np.zeros(n, np.int32)
-        t = np.zeros(n, np.float32)
-        u = np.zeros(n, np.float32)
-        v = np.zeros(n, np.float32)
+        prim = np.empty(n, np.int32)
+        t = np.empty(n, np.float32)
+        u = np.empty(n, np.float32)
+        v = np.empty(n, np.float32)
         self._check(self.lib.tt_intersect_batch(self.h, _fp(rays), n, prim.ctypes.data_as(C.POINTER(C.c_int32)),
                                                 _fp(t), _fp(u), _fp(v)), "tt_intersect_batch")
         return prim, t, u, v
 
     def occluded(self, rays: np.ndarray):
         rays = np.ascontiguousarray(rays, dtype=np.float32).reshape(-1, 8)
-        out = np.zeros(len(rays), np.uint8)
+        out = np.empty(len(rays), np.uint8)
         self._check(self.lib.tt_occluded_batch(self.h, _fp(rays), len(rays), out.ctypes.data_as(C.POINTER(C.c_uint8))),
                     "tt_occluded_batch")
-        return out.astype(bool)
+        return out.view(bool)
 
     def count_traversal(self, rays: np.ndarray):
         rays = np.ascontiguousarray(rays, dtype=np.float32).reshape(-1, 8)
@@ -300,7 +300,7 @@ class GpuContext:
         """views: [(CameraSpec, spp)].  Returns one (yres, xres, 3) linear float image per
         view (row 0 at the bottom, as framebuffer())."""
         arr, npix = self._views(views)
-        rgb = np.zeros(3 * npix, np.float32)
+        rgb = np.empty(3 * npix, np.float32)
         self._check(self.lib.tt_render_views(self.h, arr, len(views), seed, _fp(rgb)), "tt_render_views")
         out, o = [], 0
         for cam, _ in views:
