@@ -1807,15 +1807,14 @@ __device__ __forceinline__ void add_emission(float3& acc, float3 emission, float
 // estimation to `shadow` (as soon as it is made: it need not stay in registers) and samples the
 // next ray into v.  guided(s, beta): a guided vertex, queued for the network.
 enum { kPathDone, kPathNext, kPathGuided };
-template <bool MEDIA, bool GUIDE, class Org, class Rr, class Shadow, class Guided>
+template <bool MEDIA, bool GUIDE, class Org, class Rr, class Emit, class Shadow, class Guided>
 __device__ __forceinline__ int shade_step(const DevScene& sc, int bounce, float4 h, float4 vol, PathVars& v, Org&& org,
-                                          Rr&& rr, Shadow&& shadow, Guided&& guided_vertex) {
+                                          Rr&& rr, Emit&& emit, Shadow&& shadow, Guided&& guided_vertex) {
   const float3 dir = v.d;
   const Lambda l = unpack_lambda(v.lam);
   float3 beta = v.beta;
   const float prev_pdf = v.pdf;
   const bool prev_delta = v.delta;
-  float3 acc = v.acc;
   Rng& rng = v.rng;
   const int count = v.count + 1;
   const int tri = __float_as_int(h.w);
@@ -1846,7 +1845,7 @@ __device__ __forceinline__ int shade_step(const DevScene& sc, int bounce, float4
       float pdf_due = prev_delta ? dfac * prev_pdf : dfac / (h.x * h.x + kEps) * prev_pdf;
       if (MEDIA) pdf_due *= ctr;
       const float mis = mis_weight(sc, pdf_due, prev_delta, pdf_direct);
-      add_emission(acc, end_weight, beta, mis);
+      emit(end_weight, beta, mis);
     }
   } else {
     // Escaped: environment emission with MIS, then the walk ends.
@@ -1854,7 +1853,7 @@ __device__ __forceinline__ int shade_step(const DevScene& sc, int bounce, float4
       const float3 end_weight = env_eval_total(sc, -dir, l);
       const float pdf_direct = env_pdf_total(sc, -dir) * sc.type_probs[0];
       const float mis = mis_weight(sc, MEDIA ? prev_pdf * ctr : prev_pdf, prev_delta, pdf_direct);
-      add_emission(acc, end_weight, beta, mis);
+      emit(end_weight, beta, mis);
     }
     done = true;
   }
@@ -1875,7 +1874,6 @@ __device__ __forceinline__ int shade_step(const DevScene& sc, int bounce, float4
       done = true;
     }
   }
-  v.acc = acc;
   if (done) return kPathDone;
   const float3 wi = -dir;
   // Guided scattering at diffuse and microfacet surfaces.
@@ -1977,11 +1975,21 @@ struct GuidedQueue {
   }
 };
 
+// Bound by the latency of the path-state loads (long scoreboard 8-11 of 18 cycles per issue) and,
+// where many shader kinds run, by instruction fetch (4 of 18).  So without media a path's
+// accumulator is touched only where emission is added (32 of about 240 bytes per vertex: Cornell
+// box 256x256 x 16 1.89 -> 1.85 ms, guided room 3.58 -> 3.46; with media, at two blocks per SM, it
+// measured 5 % slower), and in scenes that sort their hits the warps of a block start each round
+// together, which keeps them near the same code (terrain x 16 44.1 -> 43.5 ms, 24 views
+// 9.46 -> 9.32; neutral to 1 % slower with one or two shader kinds).
 template <bool MEDIA>
 __global__ void __launch_bounds__(256, MEDIA ? 2 : 3) k_shade(DevScene sc, PathState p, int bounce) {
   const int n = *ext_count(p, bounce);
   const int* q = sorted_bounce(sc, p, bounce) ? p.sort_q : p.ext_q[bounce & 1];
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+  for (int i0 = blockIdx.x * blockDim.x; i0 < n; i0 += gridDim.x * blockDim.x) {
+    if (sc.sort_shading) __syncthreads();  // uniform
+    const int i = i0 + threadIdx.x;
+    if (i >= n) continue;
     const int slot = q[i];
     const float4 h = p.hit[slot];
     uint4 meta = p.meta[slot];
@@ -1990,7 +1998,7 @@ __global__ void __launch_bounds__(256, MEDIA ? 2 : 3) k_shade(DevScene sc, PathS
     v.d = xyz(p.ray_d[slot]);
     v.beta = xyz(b4);
     v.pdf = b4.w;
-    v.acc = xyz(p.accum[slot]);
+    if (MEDIA) v.acc = xyz(p.accum[slot]);
     v.rng = Rng{p.rng_state[slot], p.rng_inc[slot]};
     v.lam = meta.y;
     v.count = (int)meta.z;
@@ -2000,6 +2008,11 @@ __global__ void __launch_bounds__(256, MEDIA ? 2 : 3) k_shade(DevScene sc, PathS
     const MTracker mt0 = v.mt;
     const int st = shade_step<MEDIA, true>(
         sc, bounce, h, vol, v, [&] { return xyz(p.ray_o[slot]); }, [&] { return p.rr[slot]; },
+        [&](float3 e, float3 b, float mis) {
+          if (!MEDIA) v.acc = xyz(p.accum[slot]);
+          add_emission(v.acc, e, b, mis);
+          if (!MEDIA) p.accum[slot] = make_float4(v.acc.x, v.acc.y, v.acc.z, 0.f);
+        },
         [&](const ShadowRay& s) { queue_shadow<MEDIA>(p, bounce + 1, slot, s); }, GuidedQueue{sc, p, bounce, slot});
     if (st != kPathDone) {
       meta.z = (unsigned)v.count;
@@ -2014,8 +2027,8 @@ __global__ void __launch_bounds__(256, MEDIA ? 2 : 3) k_shade(DevScene sc, PathS
       p.beta[slot] = make_float4(v.beta.x, v.beta.y, v.beta.z, v.pdf);
       p.meta[slot] = meta;
     }
-    p.accum[slot] = make_float4(v.acc.x, v.acc.y, v.acc.z, 0.f);
-    p.rng_state[slot] = v.rng.state;
+    if (MEDIA) p.accum[slot] = make_float4(v.acc.x, v.acc.y, v.acc.z, 0.f);
+    if (st != kPathDone || sc.guide_record) p.rng_state[slot] = v.rng.state;
     if (st == kPathDone) {
       const int qd = warp_append(done_count(p, bounce + 1));
       p.done_q[qd] = slot;
@@ -2674,7 +2687,8 @@ __global__ void __launch_bounds__(kPathBlock, MEDIA ? 4 : 5)
         rounded(vol.z);
         rounded(vol.w);
       }
-      ended = shade_step<MEDIA, false>(sc, bounce, h, vol, v, [&] { return v.o; }, [&] { return rr; }, take_shadow,
+      ended = shade_step<MEDIA, false>(sc, bounce, h, vol, v, [&] { return v.o; }, [&] { return rr; },
+                                       [&](float3 e, float3 b, float mis) { add_emission(v.acc, e, b, mis); }, take_shadow,
                                        NoGuide{}) == kPathDone;
       rounded(sh);
       rounded(v.acc);
