@@ -1145,6 +1145,8 @@ tt_status tt_upload_scene(tt_ctx* c) {
   }
   s.media = (const DevMedium*)upload(dmed.data(), dmed.size() * sizeof(DevMedium));
   s.num_media = (int)dmed.size();
+  s.atmosphere = 0;
+  for (const DevMedium& m : dmed) s.atmosphere |= m.kind == TT_MEDIUM_ATMOSPHERE ? 1 : 0;
   s.cam_track = make_uint2(0xffffffffu, (unsigned)-1);
   // Area lights: every triangle of an emissive material, in triangle order
   // (Scene::UpdateEmissiveIndexOffset numbers emissive primitives consecutively).

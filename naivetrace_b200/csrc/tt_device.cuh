@@ -1310,8 +1310,28 @@ __device__ __forceinline__ void history_probabilities(float3 w, float3 a, float3
   if (norm > 0.f) { *pa /= norm; *pb /= norm; } else { *pa = *pb = 0.5f; }
 }
 
-// SpectralTracking (media_integrator.cxx:90-147) against the segment majorant; the weight
-// starts at `initial`, as in the reference.  At most 999 collisions.
+// SpectralTracking (media_integrator.cxx:90-147) against the segment majorant `maj` (mfp = 1 /
+// maj) at most 999 collisions long; the weight starts at the ray's weight so far, as in the
+// reference.  One step of it: advances out.t to the next tentative collision and returns true when
+// the segment is done (out.t beyond len, or a real collision).
+__device__ __forceinline__ bool atm_track_step(const DevMedium& m, float3 org, float3 dir, float len, float maj,
+                                               float mfp, InteractionSample& out, Rng& rng, Lambda l) {
+  out.t -= logf(rng.uniform()) * mfp;
+  if (out.t > len) return true;
+  float3 ss, st;
+  atm_coeffs(m, atm_altitude(m, org + dir * out.t), l, &ss, &st);
+  const float3 sn = f3(fmaxf(0.f, maj - st.x), fmaxf(0.f, maj - st.y), fmaxf(0.f, maj - st.z));
+  float pt, pn;
+  history_probabilities(out.weight, ss, sn, &pt, &pn);
+  if (rng.uniform() < pt) {
+    out.weight = out.weight * (mfp / pt);
+    out.sigma_s = ss;
+    return true;
+  }
+  out.weight = mul(out.weight, sn) * (mfp / pn);
+  return false;
+}
+constexpr int kAtmSteps = 999;
 __device__ __forceinline__ InteractionSample atm_tracking(const DevMedium& m, float3 org, float3 dir, float len,
                                                           float3 initial, Rng& rng, Lambda l) {
   InteractionSample out;
@@ -1324,21 +1344,8 @@ __device__ __forceinline__ InteractionSample atm_tracking(const DevMedium& m, fl
     return out;
   }
   const float mfp = 1.f / maj;
-  for (int it = 1; it < 1000; ++it) {
-    out.t -= logf(rng.uniform()) * mfp;
-    if (out.t > len) return out;
-    float3 ss, st;
-    atm_coeffs(m, atm_altitude(m, org + dir * out.t), l, &ss, &st);
-    const float3 sn = f3(fmaxf(0.f, maj - st.x), fmaxf(0.f, maj - st.y), fmaxf(0.f, maj - st.z));
-    float pt, pn;
-    history_probabilities(out.weight, ss, sn, &pt, &pn);
-    if (rng.uniform() < pt) {
-      out.weight = out.weight * (mfp / pt);
-      out.sigma_s = ss;
-      return out;
-    }
-    out.weight = mul(out.weight, sn) * (mfp / pn);
-  }
+  for (int it = 0; it < kAtmSteps; ++it)
+    if (atm_track_step(m, org, dir, len, maj, mfp, out, rng, l)) return out;
   return out;
 }
 

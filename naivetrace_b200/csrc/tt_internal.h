@@ -140,6 +140,7 @@ struct DevScene {
   int num_vol_tris;
   int num_spheres;            // spheres share the BVH slot arrays (tt_bvh.h)
   int num_media;
+  int atmosphere;             // 1: one of the media is an atmosphere (host-side choice of kernels)
   const DevMedium* media;
   uint2 cam_track;            // medium tracker at the camera position
   // Learned guiding (tt_guide.cuh): sample diffuse and microfacet surfaces by one-sample
