@@ -93,15 +93,26 @@ __global__ void k_prim_boxes(BuildInput in, const uint32_t* set, uint32_t n, Aab
       hi[k] = max(hi[k], ordered(c[k]));
     }
   }
+  // One atomic per bound and block: one per warp serialised on the six addresses (161 us of the
+  // build of 2.75 M primitives).
+  __shared__ unsigned part[6][kThreads / 32];
   for (int k = 0; k < 3; ++k) {
     for (int o = 16; o > 0; o >>= 1) {
       lo[k] = min(lo[k], __shfl_xor_sync(0xffffffffu, lo[k], o));
       hi[k] = max(hi[k], __shfl_xor_sync(0xffffffffu, hi[k], o));
     }
     if ((threadIdx.x & 31) == 0) {
-      atomicMin(&cbounds[k], lo[k]);
-      atomicMax(&cbounds[3 + k], hi[k]);
+      part[k][threadIdx.x >> 5] = lo[k];
+      part[3 + k][threadIdx.x >> 5] = hi[k];
     }
+  }
+  __syncthreads();
+  if (threadIdx.x < 6) {
+    unsigned v = part[threadIdx.x][0];
+    for (int w = 1; w < kThreads / 32; ++w)
+      v = threadIdx.x < 3 ? min(v, part[threadIdx.x][w]) : max(v, part[threadIdx.x][w]);
+    if (threadIdx.x < 3) atomicMin(&cbounds[threadIdx.x], v);
+    else atomicMax(&cbounds[threadIdx.x], v);
   }
 }
 
@@ -203,12 +214,133 @@ __global__ void k_merge(const int* clusters, int c, const int* nn, const int* cr
   }
 }
 
+// The clustering iterations from at most kTailClusters clusters down to one, in one block: the
+// clusters' boxes, ids and neighbours in shared memory, thread t owning clusters 4t .. 4t + 3 so
+// that the scans run in cluster order.  The pairs, node numbers and cluster order are those of the
+// kernels above; an iteration costs a few microseconds instead of nine launches, four copies and a
+// synchronisation (50-60 us), and about half of a build's 46 iterations (2.75 M primitives) start
+// with so few clusters.  ranges[i]: first node and node count of iteration i; info: iterations
+// done, next node, the last cluster's node, 1 when an iteration made no progress.
+constexpr int kTailThreads = 1024, kTailEach = 4, kTailClusters = kTailThreads * kTailEach;
+constexpr int kTailSmem = kTailClusters * (int)(sizeof(Aabb) + 2 * sizeof(int));
+__global__ void __launch_bounds__(kTailThreads) k_cluster_tail(const int* clusters, int c, int radius, int next_node,
+                                                               int total, int max_iterations, Aabb* node_box,
+                                                               int* left, int* right, int2* ranges, int* info) {
+  extern __shared__ __align__(16) unsigned char tail_smem[];
+  Aabb* box = reinterpret_cast<Aabb*>(tail_smem);
+  int* id = reinterpret_cast<int*>(box + kTailClusters);
+  int* nn = id + kTailClusters;
+  __shared__ int wsum[2][kTailThreads / 32];
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  for (int i = t; i < c; i += kTailThreads) {
+    id[i] = clusters[i];
+    box[i] = node_box[id[i]];
+  }
+  __syncthreads();
+  int it = 0;
+  bool stuck = false;
+  while (c > 1 && it < max_iterations) {
+    for (int i = t; i < c; i += kTailThreads) {
+      const Aabb bi = box[i];
+      float best = INFINITY;
+      int bj = -1;
+      const int j0 = max(0, i - radius), j1 = min(c - 1, i + radius);
+      for (int j = j0; j <= j1; ++j) {
+        if (j == i) continue;
+        const float a = half_area(merge(bi, box[j]));
+        if (bj < 0 || pair_less(a, min(i, j), max(i, j), best, min(i, bj), max(i, bj))) {
+          best = a;
+          bj = j;
+        }
+      }
+      nn[i] = bj;
+    }
+    __syncthreads();
+    // This thread's clusters after the merge (in registers), and how many nodes and clusters it makes.
+    Aabb nb[kTailEach];
+    int nid[kTailEach], partner[kTailEach];
+    int made = 0, kept = 0;
+#pragma unroll
+    for (int e = 0; e < kTailEach; ++e) {
+      const int i = kTailEach * t + e;
+      nid[e] = -1;
+      partner[e] = -1;
+      if (i < c) {
+        const int j = nn[i];
+        const bool mutual = j >= 0 && nn[j] == i;
+        if (!(mutual && i > j)) {
+          nid[e] = id[i];
+          nb[e] = box[i];
+          ++kept;
+          if (mutual) {
+            partner[e] = id[j];
+            nb[e] = merge(nb[e], box[j]);
+            ++made;
+          }
+        }
+      }
+    }
+    int smade = made, skept = kept;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int a = __shfl_up_sync(0xffffffffu, smade, o), b = __shfl_up_sync(0xffffffffu, skept, o);
+      if (lane >= o) {
+        smade += a;
+        skept += b;
+      }
+    }
+    if (lane == 31) {
+      wsum[0][warp] = smade;
+      wsum[1][warp] = skept;
+    }
+    __syncthreads();
+    int all_made = 0, all_kept = 0, node = smade - made, out = skept - kept;
+    for (int w = 0; w < kTailThreads / 32; ++w) {
+      if (w < warp) {
+        node += wsum[0][w];
+        out += wsum[1][w];
+      }
+      all_made += wsum[0][w];
+      all_kept += wsum[1][w];
+    }
+    if (all_made == 0 || next_node + all_made > total) {  // uniform
+      stuck = true;
+      break;
+    }
+#pragma unroll
+    for (int e = 0; e < kTailEach; ++e) {
+      if (nid[e] < 0) continue;
+      if (partner[e] >= 0) {
+        const int k = next_node + node++;
+        node_box[k] = nb[e];
+        left[k] = nid[e];
+        right[k] = partner[e];
+        nid[e] = k;
+      }
+      id[out] = nid[e];
+      box[out] = nb[e];
+      ++out;
+    }
+    if (t == 0) ranges[it] = make_int2(next_node, all_made);
+    next_node += all_made;
+    c = all_kept;
+    ++it;
+    __syncthreads();
+  }
+  if (t == 0) {
+    info[0] = it;
+    info[1] = next_node;
+    info[2] = id[0];
+    info[3] = stuck || c > 1 ? 1 : 0;
+  }
+}
+
 // Bottom-up over one creation range: subtree sizes and SAH costs (traversal step 1,
 // primitive test 1 per primitive), whether a subtree of at most kMaxLeaf primitives is
 // cheaper as one leaf, and the number of inner nodes the subtree emits.
-__global__ void k_costs(int first, int count, uint32_t n, const Aabb* node_box, const int* left, const int* right,
-                        int* size, float* cost, unsigned char* collapse, int* inner) {
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < count; t += gridDim.x * blockDim.x) {
+__device__ __forceinline__ void costs_range(int start, int step, int first, int count, uint32_t n, const Aabb* node_box,
+                                            const int* left, const int* right, int* size, float* cost,
+                                            unsigned char* collapse, int* inner) {
+  for (int t = start; t < count; t += step) {
     const int k = first + t;
     const int l = left[k], r = right[k];
     const int sl = l < (int)n ? 1 : size[l], sr = r < (int)n ? 1 : size[r];
@@ -226,15 +358,33 @@ __global__ void k_costs(int first, int count, uint32_t n, const Aabb* node_box, 
   }
 }
 
+__global__ void k_costs(int first, int count, uint32_t n, const Aabb* node_box, const int* left, const int* right,
+                        int* size, float* cost, unsigned char* collapse, int* inner) {
+  costs_range(blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, first, count, n, node_box, left, right,
+              size, cost, collapse, inner);
+}
+// The small ranges of the clustering tail one after the other in one block.
+__global__ void __launch_bounds__(kTailThreads) k_costs_tail(const int2* ranges, int count, uint32_t n,
+                                                             const Aabb* node_box, const int* left, const int* right,
+                                                             int* size, float* cost, unsigned char* collapse,
+                                                             int* inner) {
+  for (int r = 0; r < count; ++r) {
+    costs_range(threadIdx.x, blockDim.x, ranges[r].x, ranges[r].y, n, node_box, left, right, size, cost, collapse,
+                inner);
+    __syncthreads();
+  }
+}
+
 // Top-down over one creation range: primitive offsets and node indices (both in depth-first
 // order: an inner node's first child follows it in memory, its second child follows the
 // first child's subtree) and whether the node is emitted as an inner node, lies inside a
 // leaf, or is a leaf itself.  state: bit 0 = inside a leaf (set by an ancestor that
 // became a leaf).
-__global__ void k_topdown(int first, int count, uint32_t n, const int* left, const int* right, const int* size,
-                          const unsigned char* collapse, const int* inner, int* offset, int* index,
-                          unsigned char* state, int* depth, unsigned char* emit, unsigned* max_depth) {
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < count; t += gridDim.x * blockDim.x) {
+__device__ __forceinline__ void topdown_range(int start, int step, int first, int count, uint32_t n, const int* left,
+                                              const int* right, const int* size, const unsigned char* collapse,
+                                              const int* inner, int* offset, int* index, unsigned char* state,
+                                              int* depth, unsigned char* emit, unsigned* max_depth) {
+  for (int t = start; t < count; t += step) {
     const int k = first + t;
     const bool inside = state[k] & 1u;
     const bool leafnode = inside || collapse[k];
@@ -252,6 +402,24 @@ __global__ void k_topdown(int first, int count, uint32_t n, const int* left, con
       index[r] = index[k] + 1 + (l < (int)n ? 0 : inner[l]);
       atomicMax(max_depth, (unsigned)(depth[k] + 1));
     }
+  }
+}
+
+__global__ void k_topdown(int first, int count, uint32_t n, const int* left, const int* right, const int* size,
+                          const unsigned char* collapse, const int* inner, int* offset, int* index,
+                          unsigned char* state, int* depth, unsigned char* emit, unsigned* max_depth) {
+  topdown_range(blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, first, count, n, left, right, size,
+                collapse, inner, offset, index, state, depth, emit, max_depth);
+}
+__global__ void __launch_bounds__(kTailThreads) k_topdown_tail(const int2* ranges, int count, uint32_t n,
+                                                               const int* left, const int* right, const int* size,
+                                                               const unsigned char* collapse, const int* inner,
+                                                               int* offset, int* index, unsigned char* state,
+                                                               int* depth, unsigned char* emit, unsigned* max_depth) {
+  for (int r = count - 1; r >= 0; --r) {
+    topdown_range(threadIdx.x, blockDim.x, ranges[r].x, ranges[r].y, n, left, right, size, collapse, inner, offset,
+                  index, state, depth, emit, max_depth);
+    __syncthreads();
   }
 }
 
@@ -367,6 +535,15 @@ __device__ void write_node4_bytes(float4* d, const Aabb* box, const int* ref, in
                      __int_as_float(ref[m > 3 ? 3 : 0]));
 }
 
+// atomicAdd(counter, 1) of every active lane, one atomic per warp.
+__device__ __forceinline__ int count_up(int* counter) {
+  const unsigned mask = __activemask();
+  const int lane = threadIdx.x & 31, leader = __ffs(mask) - 1;
+  int base = 0;
+  if (lane == leader) base = atomicAdd(counter, __popc(mask));
+  return __shfl_sync(mask, base, leader) + __popc(mask & ((1u << lane) - 1u));
+}
+
 // 4-wide layout, built top down one level at a time: a 4-wide node starts from a binary
 // inner node's two children and, while it has fewer than four, replaces the inner child of
 // the largest surface area by that child's two children (the usual collapse of a binary
@@ -406,8 +583,8 @@ __global__ void k_collapse4(const int4* frontier, int nfront, uint32_t n, const 
       const int c = slot[j];
       box[j] = node_box[c];
       if (c >= (int)n && emit[c]) {
-        const int j4 = atomicAdd(counter, 1);
-        next[atomicAdd(nnext, 1)] = make_int4(c, j4, frontier[t].z + m - 1, 0);
+        const int j4 = count_up(counter);
+        next[count_up(nnext)] = make_int4(c, j4, frontier[t].z + m - 1, 0);
         ref[j] = j4;
       } else {
         ref[j] = child_ref(c, n, size, offset, emit, index);
@@ -415,7 +592,7 @@ __global__ void k_collapse4(const int4* frontier, int nfront, uint32_t n, const 
     }
     if (bytes) write_node4_bytes(nodes4 + 4 * (size_t)i4, box, ref, m);
     else write_node4_float(nodes4 + 8 * (size_t)i4, box, ref, m);
-    atomicMax(stack_need, frontier[t].z + 4);
+    if (frontier[t].z + 4 > *(volatile int*)stack_need) atomicMax(stack_need, frontier[t].z + 4);
   }
 }
 // 4-wide root of a tree whose root is a leaf: one slot with the leaf.
@@ -557,7 +734,7 @@ bool device_build_bvh2(const BuildInput& in, const uint32_t* set, uint32_t n, De
   int iterations = 0;
   const char* radius_env = std::getenv("TT_PLOC_RADIUS");
   const int radius = radius_env ? std::max(1, std::min(256, std::atoi(radius_env))) : kDefaultRadius;
-  while (c > 1) {
+  while (c > kTailClusters) {
     if (++iterations > kMaxIterations) return fail("clustering did not converge");
     k_nearest<<<grid_for(c), kThreads, 0, st>>>(cur, c, node_box, radius, nn);
     k_merge_flags<<<grid_for(c), kThreads, 0, st>>>(nn, c, create, keep);
@@ -580,11 +757,21 @@ bool device_build_bvh2(const BuildInput& in, const uint32_t* set, uint32_t n, De
     c = kept;
     std::swap(cur, nxt);
   }
-  const double t_clustered = verbose ? ms_since(t_start) : 0.0;
-  if (!ok(cudaMemcpyAsync(&hb[4], cur, sizeof(int), cudaMemcpyDeviceToHost, st), "copy") ||
-      !ok(cudaStreamSynchronize(st), "sync"))
+  // The rest in one block.
+  int2* tail_ranges = sc.alloc<int2>(kMaxIterations);
+  int* tail_info = sc.alloc<int>(4);
+  if (!tail_ranges || !tail_info) return fail("out of device memory");
+  if (!ok(cudaFuncSetAttribute(k_cluster_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailSmem), "attribute"))
     return false;
-  const int root = hb[4];
+  k_cluster_tail<<<1, kTailThreads, kTailSmem, st>>>(cur, c, radius, next_node, (int)total, kMaxIterations - iterations,
+                                                     node_box, left, right, tail_ranges, tail_info);
+  if (!ok(cudaMemcpyAsync(&hb[20], tail_info, 4 * sizeof(int), cudaMemcpyDeviceToHost, st), "copy") ||
+      !ok(cudaStreamSynchronize(st), "clustering"))
+    return false;
+  const int tail_count = hb[20], root = hb[22];
+  if (hb[23] != 0) return fail("clustering made no progress or did not converge");
+  iterations += tail_count;
+  const double t_clustered = verbose ? ms_since(t_start) : 0.0;
   // Bottom-up costs, top-down offsets and emission.
   int* size = sc.alloc<int>(total);
   float* cost = sc.alloc<float>(total);
@@ -604,10 +791,13 @@ bool device_build_bvh2(const BuildInput& in, const uint32_t* set, uint32_t n, De
   for (const auto& r : ranges)
     k_costs<<<grid_for(r.second), kThreads, 0, st>>>(r.first, r.second, n, node_box, left, right, size, cost, collapse,
                                                       inner);
+  k_costs_tail<<<1, kTailThreads, 0, st>>>(tail_ranges, tail_count, n, node_box, left, right, size, cost, collapse, inner);
   cudaMemsetAsync(offset + root, 0, sizeof(int), st);
   cudaMemsetAsync(index + root, 0, sizeof(int), st);
   cudaMemsetAsync(state + root, 0, 1, st);  // no state
   cudaMemsetAsync(depth + root, 0, sizeof(int), st);
+  k_topdown_tail<<<1, kTailThreads, 0, st>>>(tail_ranges, tail_count, n, left, right, size, collapse, inner, offset,
+                                             index, state, depth, emit, max_depth);
   for (auto it = ranges.rbegin(); it != ranges.rend(); ++it)
     k_topdown<<<grid_for(it->second), kThreads, 0, st>>>(it->first, it->second, n, left, right, size, collapse, inner,
                                                           offset, index, state, depth, emit, max_depth);
@@ -638,8 +828,7 @@ bool device_build_bvh2(const BuildInput& in, const uint32_t* set, uint32_t n, De
     k_leaf_root<<<1, 1, 0, st>>>(node_box, root, (int)n, out->nodes);
     k_leaf_root4<<<1, 1, 0, st>>>(node_box, root, (int)n, out->nodes4);
   } else {
-    for (const auto& r : ranges)
-      k_write_nodes<<<grid_for(r.second), kThreads, 0, st>>>(r.first, r.second, n, node_box, left, right, size, offset,
+    k_write_nodes<<<grid_for(total - n), kThreads, 0, st>>>((int)n, (int)(total - n), n, node_box, left, right, size, offset,
                                                               emit, index, out->nodes);
     int4* front[2] = {sc.alloc<int4>(cap4), sc.alloc<int4>(cap4)};
     int* counts = sc.alloc<int>(3);  // [0] 4-wide nodes numbered, [1] next level's size, [2] stack entries needed

@@ -80,3 +80,17 @@ def test_renders_on_every_layout(algo, name, monkeypatch):
     assert np.array_equal(images[0], images[1])
     # The 8-wide layout's own boxes may decide a grazing ray otherwise.
     assert np.isclose(images[0], images[2], rtol=1e-5, atol=1e-6).mean() > 0.999
+
+
+@pytest.mark.parametrize("prims", [1, 2, 3, 5, 4095, 4096, 4097, 9001])
+def test_device_build_equals_host_build(prims, monkeypatch):
+    """Around the cluster count where the device build goes on in one block: the same hits as on
+    the host-built tree."""
+    scene = _heightfield(prims, min(2, prims - 1), 0.0)
+    device = GpuContext(scene, make_params())
+    monkeypatch.setenv("TT_BVH_BUILD", "host")
+    host = GpuContext(scene, make_params())
+    rays = _rays(60001, 0.0)
+    for a, b in zip(device.intersect(rays), host.intersect(rays)):
+        assert np.array_equal(a, b)
+    assert np.array_equal(device.occluded(rays), host.occluded(rays))
