@@ -287,6 +287,7 @@ class CountAreas {
       if (!kept().empty()) {
         unsigned long long* p = kept().back();
         kept().pop_back();
+        std::memset(p, 0, kEntries * sizeof(unsigned long long));  // no report of an earlier context's wave
         return p;
       }
     }
@@ -296,6 +297,7 @@ class CountAreas {
       cudaGetLastError();
       return nullptr;
     }
+    std::memset(p, 0, kEntries * sizeof(unsigned long long));
     return static_cast<unsigned long long*>(p);
   }
   static void give(unsigned long long* p) {
@@ -2680,6 +2682,7 @@ static tt_status render_views(tt_ctx* c, const tt_view* views, int32_t n, uint64
   ++done_waves;
   if ((st = check(cudaGetLastError())) != TT_OK) return st;
   if (nwaves > 1) {
+    prepare_paths_launch(sc);
     if ((st = check(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal))) != TT_OK) return st;
     const int per_wave = wave(c->stream, false);
     cudaError_t ce = cudaStreamEndCapture(c->stream, &graph);

@@ -297,6 +297,8 @@ void launch_gather(const PathState& p, const Framebuffer& fb, const WaveArgs& w,
 enum { kFlushNone = 0, kFlushNow = 1, kFlushCaptured = 2 };
 bool launch_paths(const DevScene& s, const PathState& p, const Framebuffer& fb, const WaveArgs& w, int first, int rounds,
                   int max_n, int flush, unsigned long long* stats, cudaStream_t st);
+// Loads launch_paths' kernels for the scene, outside stream capture.
+void prepare_paths_launch(const DevScene& s);
 // Guided scenes: network evaluation and one-sample MIS scattering of the queued guided
 // vertices (persistent kernel, as many CTAs as fit on the SMs).
 void launch_guide(const DevScene& s, const PathState& p, int bounce, cudaStream_t st);

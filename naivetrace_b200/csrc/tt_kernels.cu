@@ -3330,20 +3330,34 @@ void launch_gather(const PathState& p, const Framebuffer& fb, const WaveArgs& w,
   });
 }
 
-bool launch_paths(const DevScene& s, const PathState& p, const Framebuffer& fb, const WaveArgs& w, int first, int rounds,
-                  int max_n, int flush, unsigned long long* stats, cudaStream_t st) {
-  if (s.algo != TT_ALGO_PT || s.wide != 0) return false;
-  const int smem = 3 * (rounds + 2) * (int)sizeof(int);
+// Calls f with the k_paths instantiation of the scene.
+template <class F>
+static void with_paths_kernel(const DevScene& s, F&& f) {
   with_bool(s.num_media > 0, [&](auto M) {
     with_bool(s.num_spheres > 0, [&](auto S) {
       with_layout(s, [&](auto W) {
         constexpr int L = decltype(W)::value;
-        if constexpr (L != kLayout8) {
-          auto* k = k_paths<decltype(M)::value, decltype(S)::value, L>;
-          k<<<full_grid(k, kPathBlock), kPathBlock, smem, st>>>(s, p, fb, w, first, rounds, max_n, flush, stats);
-        }
+        if constexpr (L != kLayout8) f(k_paths<decltype(M)::value, decltype(S)::value, L>);
       });
     });
+  });
+}
+
+void prepare_paths_launch(const DevScene& s) {
+  cudaFuncAttributes a;
+  with_paths_kernel(s, [&](auto* k) {
+    full_grid(k, kPathBlock);
+    cudaFuncGetAttributes(&a, k);
+  });
+  cudaFuncGetAttributes(&a, k_paths_taken);
+}
+
+bool launch_paths(const DevScene& s, const PathState& p, const Framebuffer& fb, const WaveArgs& w, int first, int rounds,
+                  int max_n, int flush, unsigned long long* stats, cudaStream_t st) {
+  if (s.algo != TT_ALGO_PT || s.wide != 0) return false;
+  const int smem = 3 * (rounds + 2) * (int)sizeof(int);
+  with_paths_kernel(s, [&](auto* k) {
+    k<<<full_grid(k, kPathBlock), kPathBlock, smem, st>>>(s, p, fb, w, first, rounds, max_n, flush, stats);
   });
   if (flush == kFlushCaptured) k_paths_taken<<<1, 32, 0, st>>>(p, first, max_n, stats);
   return true;
