@@ -1558,16 +1558,28 @@ static tt_status guide_train(tt_ctx* c, long long paths) {
   return TT_OK;
 }
 
-// A wave runs as whole paths in one launch from its camera samples up to kWholePaths, and from
-// the bounce on where at most kTailPaths are left.  k_paths serves few paths at the latency of one
-// path's stages; with many it is 2-4 times slower than the wavefront kernels (96-128 registers with
-// spills, every lane in its own material).  64x64 pixels, k_paths against the wavefront: Cornell
-// box 0.17 / 0.49 ms at 1 sample, 0.50 / 0.65 at 32 (131,072 paths); with medium 0.53 / 1.72 and
-// 2.28 / 2.47; terrain 0.34 / 1.26 and 1.93 / 2.75.  Tail limits of 4,096 / 32,768 / 65,536 /
-// 262,144 paths: terrain 641x359 x 1 2.23 / 1.81 / 1.75 / 1.95 ms (3.25 without), medium box
-// 512x512 x 8 8.11 / 8.06 / 8.09 / 8.27 (8.39), planet 7.12 / 6.97 / 6.99 / 7.06 (8.48).
-constexpr int kWholePaths = 1 << 17;
-constexpr int kTailPaths = 1 << 16;
+// A wave runs as whole paths in one launch from its camera samples up to whole_paths(), and from
+// the bounce on where at most tail_paths() are left.  k_paths serves few paths at the latency of
+// one path's stages; with many it is up to 4 times slower than the wavefront kernels (96-128
+// registers with spills, every lane in its own material, no queue between walk and shading).  How
+// many are few depends on what the lanes of a warp share: in a scene without media whose hits are
+// not sorted for shading they shade alike (uniform), and in a BVH below the byte boxes' size they
+// walk alike.  128x128 pixels, us per pass, k_paths from the camera / wavefront with tail:
+//   Cornell box    16k paths 122 / 173 (depth 4), 330 / 378 (20); 64k 156 / 205, 451 / 500
+//   furnished room 16k paths 117 / 141, 395 / 427;                64k 128 / 152, 489 / 514
+//   terrain        16k paths 281 / 314, 351 / 379;                32k 406 / 332, 521 / 423
+//   materials      16k paths 232 / 238, 667 / 666;                32k 309 / 261, 926 / 808
+//   medium         16k paths 256 / 256, 841 / 837;                32k 297 / 271, 1087 / 983
+// and at 128k paths it loses in the room too (741 / 695 at depth 20).  Tail limits of 16k / 64k
+// paths, depth 20, 64k paths in the wave: Cornell box 604 / 500, terrain 535 / 449, room 577 /
+// 514; materials 966 / 1207, medium 1158 / 1269, spheres 981 / 1069, media mix 1885 / 2093.
+constexpr int kFewPaths = 1 << 14;
+constexpr int kFewUniformPaths = 1 << 16;
+static bool uniform_shading(const DevScene& s) { return s.num_media == 0 && s.sort_shading == 0; }
+static int whole_paths(const DevScene& s) {
+  return uniform_shading(s) && !s.nodes4_bytes ? kFewUniformPaths : kFewPaths;
+}
+static int tail_paths(const DevScene& s) { return uniform_shading(s) ? kFewUniformPaths : kFewPaths; }
 
 // Starts a new wave's queue-length reports.
 static void next_wave_tag(tt_ctx* c) {
@@ -1651,7 +1663,7 @@ static tt_status render_range(tt_ctx* c, int32_t spp, uint64_t seed, int32_t pb,
     // bounces' few paths as whole paths again (after the guided bounces).  Not with guiding
     // records, nor when single launches are timed or counted.
     const bool whole = !c->dev.guide_record && !timing && c->dev.algo == TT_ALGO_PT && !c->dev.wide;
-    const bool fused = whole && !c->dev.guide && w.wave_paths <= kWholePaths &&
+    const bool fused = whole && !c->dev.guide && w.wave_paths <= whole_paths(c->dev) &&
                        launch_paths(c->dev, c->ps, c->fb, w, -1, rounds, INT_MAX, kFlushNone, c->d_stats, c->stream);
     if (!fused) {
       if (whole) next_wave_tag(c);
@@ -1665,7 +1677,7 @@ static tt_status render_range(tt_ctx* c, int32_t spp, uint64_t seed, int32_t pb,
         ++shadow_launches;
         if (c->dev.guide_record) launch_flush(c->dev, c->ps, c->fb, b, grid, c->stream);
         // The launches of bounce b - 1 keep the device busy while the host reads its count.
-        if (c->ps.host_counts && b >= tail && reported_count(c, b - 1) <= (unsigned)kTailPaths &&
+        if (c->ps.host_counts && b >= tail && reported_count(c, b - 1) <= (unsigned)tail_paths(c->dev) &&
             launch_paths(c->dev, c->ps, c->fb, w, b, rounds, INT_MAX, kFlushNone, c->d_stats, c->stream)) {
           launches += 2;
           break;
@@ -2646,13 +2658,13 @@ static tt_status render_views(tt_ctx* c, const tt_view* views, int32_t n, uint64
       launch_flush(sc, ps, fb, b, grid, s);
       k += 2;
       if (eager) {
-        if (ps.host_counts && b >= tail && reported_count(c, b - 1) <= (unsigned)kTailPaths &&
+        if (ps.host_counts && b >= tail && reported_count(c, b - 1) <= (unsigned)tail_paths(sc) &&
             launch_paths(sc, ps, fb, none, b, rounds, INT_MAX, kFlushNow, c->d_stats, s)) {
           ++k;
           break;
         }
       } else if (whole && b >= tail && b % 4 == 0 &&
-                 launch_paths(sc, ps, fb, none, b, rounds, kTailPaths, kFlushCaptured, c->d_stats, s)) {
+                 launch_paths(sc, ps, fb, none, b, rounds, tail_paths(sc), kFlushCaptured, c->d_stats, s)) {
         k += 2;
       }
       launch_extend(sc, ps, b, false, nullptr, grid, s);

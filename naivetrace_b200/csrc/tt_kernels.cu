@@ -2666,7 +2666,7 @@ struct NoGuide {
 // triangles, 100-180 us on the terrain); here that chain is paid once per path: a
 // 64x64 box at one sample takes 0.17 ms instead of 0.49 ms.  What bounds it is the issue of one
 // warp's instruction stream (6-7 cycles each at one warp per scheduler); when it serves how many
-// paths is in tt_capi.cu (kWholePaths, kTailPaths).
+// paths is in tt_capi.cu (whole_paths, tail_paths).
 // The stages are the wavefront kernels' functions in their order per path, so the results are the
 // same.  first < 0: the wave's camera samples, the finished paths' RGB left in accum for k_gather;
 // else the paths of bounce `first`'s extension queue (their shadow rays of that bounce traced

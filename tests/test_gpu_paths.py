@@ -9,7 +9,9 @@ from naivetrace_b200.scene import make_params
 
 pytestmark = pytest.mark.gpu
 
-WHOLE = 1 << 17  # paths up to which a wave runs as whole paths from its camera samples
+# Paths up to which a wave runs as whole paths from its camera samples: in any scene, and in a small
+# uniform one (also the limits of the last bounces' paths).
+WHOLE, WHOLE_UNIFORM = 1 << 14, 1 << 16
 
 
 def _render(scene, params, spp, wavefront, rng=None, guide=False):
@@ -53,10 +55,16 @@ def test_whole_paths(name, xres, yres, spp):
 
 
 @pytest.mark.parametrize("name", sorted(SCENES))
-@pytest.mark.parametrize("spp", [31, 32, 33])  # 64 x 64 x 32 = WHOLE
+@pytest.mark.parametrize("spp", [3, 4, 5, 31, 32, 33])  # 64 x 64 x 4 = WHOLE
 def test_around_the_limit(name, spp):
-    assert 64 * 64 * 32 == WHOLE
+    assert 64 * 64 * 4 == WHOLE
     _same(SCENES[name](64, 64), make_params(max_ray_depth=12), spp)
+
+
+@pytest.mark.parametrize("spp", [15, 16, 17])  # 64 x 64 x 16 = WHOLE_UNIFORM
+def test_around_the_uniform_limit(spp):
+    assert 64 * 64 * 16 == WHOLE_UNIFORM
+    _same(scenes.cornell_box(64, 64), make_params(max_ray_depth=12), spp)
 
 
 @pytest.mark.parametrize("depth", [1, 2, 3, 1000])
