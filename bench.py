@@ -611,7 +611,6 @@ def run_ours(args):
         step()
     g.clear()
     g.reset_stats()
-    g.set_profiling(1)
     clocks = ClockSampler(device)
     nd.barrier(r)
     torch.cuda.synchronize()
@@ -627,16 +626,23 @@ def run_ours(args):
     clk = clocks.stop()
     elapsed_ms = ev0.elapsed_time(ev1)
     st = g.stats()
+    # One more frame with every closest-hit and shadow launch timed (all bounces then run as
+    # wavefront launches) for the kernels' own rates.
+    g.reset_stats()
+    g.set_profiling(1)
+    step()
+    torch.cuda.synchronize()
+    sp = g.stats()
     g.set_profiling(0)
     elapsed_ms = nd.max_over_ranks(elapsed_ms, r)
     ms_per_step = elapsed_ms / args.steps
     value = nd.weak_scaling_value(paths_per_step, world, ms_per_step)
     mrays = world * (st["extension_rays"] + st["shadow_rays"]) / args.steps / (ms_per_step * 1e-3) / 1e6
     # Roofline of the dominant kernel (closest-hit traversal).
-    ext_launch_ms = st["extend_ms"] / max(st["extend_launches"], 1)
-    achieved_gbs = st["extension_rays"] * bytes_per_ray / (st["extend_ms"] * 1e-3) / 1e9 if st["extend_ms"] > 0 else 0.0
+    ext_launch_ms = sp["extend_ms"] / max(sp["extend_launches"], 1)
+    achieved_gbs = sp["extension_rays"] * bytes_per_ray / (sp["extend_ms"] * 1e-3) / 1e9 if sp["extend_ms"] > 0 else 0.0
     peak, peak_kind = hbm_peak()
-    rays_per_launch = st["extension_rays"] / max(st["extend_launches"], 1)
+    rays_per_launch = sp["extension_rays"] / max(sp["extend_launches"], 1)
     traffic = None
     tfile = ROOT / "profiles" / "extend_traffic.json"
     if tfile.exists():
@@ -741,9 +747,10 @@ def run_ours(args):
             "sorted_shading": sorted_shading,
             "gpu_launches": int(st["kernel_launches"]),
             "clocks": clk,
-            "stats": {k: st[k] for k in ("extension_rays", "shadow_rays", "extend_launches", "extend_ms",
-                                         "shadow_launches", "shadow_ms", "pass_ms", "bvh_nodes", "bvh_depth",
-                                         "error_flags")},
+            "stats": {k: st[k] for k in ("extension_rays", "shadow_rays", "extend_launches", "shadow_launches",
+                                         "pass_ms", "bvh_nodes", "bvh_depth", "error_flags")},
+            "profiled_frame": {k: sp[k] for k in ("extension_rays", "shadow_rays", "extend_launches", "extend_ms",
+                                                  "shadow_launches", "shadow_ms", "pass_ms")},
         }
         print(json.dumps(line))
     g.close()
