@@ -233,7 +233,7 @@ typedef struct tt_stats {
   uint64_t paths;               /* camera samples started */
   uint64_t extension_rays;      /* closest-hit queries */
   uint64_t shadow_rays;         /* occlusion queries */
-  uint64_t extend_launches;     /* closest-hit kernel launches */
+  uint64_t extend_launches;     /* closest-hit kernel launches (whole paths in one launch not among them) */
   double extend_ms;             /* summed CUDA-event time of those launches (if profiling) */
   uint64_t shadow_launches;
   double shadow_ms;
@@ -386,7 +386,9 @@ tt_status tt_read_accumulators_device(tt_ctx* ctx, double* d_accum, double* d_li
 
 /* Profiling level: 0 off; 1 render passes time each closest-hit and shadow launch with
  * CUDA events on the launching stream and add the durations to the stats; 2 additionally
- * counts BVH nodes visited and triangles tested (slower; for the bytes-per-ray model). */
+ * counts BVH nodes visited and triangles tested (slower; for the bytes-per-ray model).  From
+ * level 1 every bounce runs as its own launches, where a pass would otherwise take small waves
+ * and the last bounces' few paths as whole paths in one launch (same results, more time). */
 tt_status tt_set_profiling(tt_ctx* ctx, int32_t on);
 tt_status tt_get_stats(tt_ctx* ctx, tt_stats* out);
 tt_status tt_reset_stats(tt_ctx* ctx);
