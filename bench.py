@@ -648,7 +648,8 @@ def run_ours(args):
     if tfile.exists():
         try:
             td = json.loads(tfile.read_text())
-            traffic = td.get("bytes_per_ray", 0) * rays_per_launch
+            if td.get("node_bytes") == cst["bvh_node_bytes"]:  # captured with another node layout: no figure
+                traffic = td["bytes_per_ray"] * rays_per_launch
         except Exception:
             traffic = None
 
