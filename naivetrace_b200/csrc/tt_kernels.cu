@@ -563,6 +563,10 @@ __device__ __forceinline__ int visit_node4_any(const float4* __restrict__ nodes4
 // when the ray meets the leaf's box in the float test (it then meets every box around it, slab
 // distances being monotone in the planes): tested on the primitive's own box, which lies in the
 // leaf's, and only if that fails on the leaf's.
+// A closest hit is not held to the nearest hit so far there (the caller passes no limit): the
+// error of a box's entry is one of the ray origin's scale, so the entry of a nearer hit's box can
+// lie behind an earlier hit of the neighbouring leaf, which the walk with float boxes, testing both
+// leaves' boxes before either's primitives, does not mind.
 template <bool SPH>
 __device__ __forceinline__ void slot_box(float4 a, float4 b, float4 c, float3& lo, float3& hi) {
   lo = f3(fminf(a.x, fminf(b.x, c.x)), fminf(a.y, fminf(b.y, c.y)), fminf(a.z, fminf(b.z, c.z)));
@@ -615,7 +619,7 @@ __device__ __forceinline__ bool test_leaf(const float4* __restrict__ tris, const
     if (SPH && __float_as_int(cc.w) != 0) hit = intersect_sphere(r, a, b, tnear, best_t, &t);
     else hit = intersect_tri(r, xyz(a), xyz(b), xyz(cc), tnear, best_t, &t, &b1, &b2);
     if (hit && (ANY || closer(t, __float_as_int(a.w), best_t, best_prim)) &&
-        (!BYTES || !check || leaf_box_met<SPH>(tris, r, start, count, a, b, cc, tnear, best_t))) {
+        (!BYTES || !check || leaf_box_met<SPH>(tris, r, start, count, a, b, cc, tnear, ANY ? best_t : INFINITY))) {
       best = i;
       best_prim = __float_as_int(a.w);
       best_t = t;
