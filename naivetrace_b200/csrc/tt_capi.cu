@@ -1685,7 +1685,7 @@ static tt_status render_range(tt_ctx* c, int32_t spp, uint64_t seed, int32_t pb,
         timed(0, [&] { launch_extend(c->dev, c->ps, b, counting, c->d_stats, grid, c->stream); });
         ++extend_launches;
         if (c->dev.num_media > 0) {
-          launch_track(c->dev, c->ps, b, grid, c->stream);
+          launch_track(c->dev, c->ps, b, w.wave_paths, grid, c->stream);
           launches++;
         }
         launch_shade(c->dev, c->ps, b, grid, c->stream);
@@ -2668,7 +2668,7 @@ static tt_status render_views(tt_ctx* c, const tt_view* views, int32_t n, uint64
         k += 2;
       }
       launch_extend(sc, ps, b, false, nullptr, grid, s);
-      if (sc.num_media > 0) launch_track(sc, ps, b, grid, s);
+      if (sc.num_media > 0) launch_track(sc, ps, b, hw[0].wave_paths, grid, s);
       launch_shade(sc, ps, b, grid, s);
       if (sc.guide && b < sc.guide_depth) launch_guide(sc, ps, b, s);
       k += 1 + (sc.num_media > 0) + shade_launches(sc, ps, b) + (sc.guide && b < sc.guide_depth);

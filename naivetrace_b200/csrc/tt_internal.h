@@ -303,7 +303,8 @@ void prepare_paths_launch(const DevScene& s);
 // vertices (persistent kernel, as many CTAs as fit on the SMs).
 void launch_guide(const DevScene& s, const PathState& p, int bounce, cudaStream_t st);
 // Media scenes: spectral tracking from each extension ray's origin to its surface hit.
-void launch_track(const DevScene& s, const PathState& p, int bounce, int grid, cudaStream_t st);
+// paths: paths of the wave (an upper bound of the bounce's queue).
+void launch_track(const DevScene& s, const PathState& p, int bounce, int paths, int grid, cudaStream_t st);
 // Medium tracker at `pos` (MediumTracker::initializePosition); writes one uint2 to `out`.
 void launch_init_tracker(const DevScene& s, float3 pos, float3 bb_lo, float3 bb_hi, uint2* out, unsigned int* err,
                          cudaStream_t st);

@@ -1741,7 +1741,12 @@ __global__ void __launch_bounds__(256) k_track(DevScene sc, PathState p, int bou
 // once kTrackRefill lanes are not, those end their segments, write their results and take new paths
 // (as the closest-hit queue does).  Per path the operations and their order are track_step's.
 // Planet 512x512 x 8: 6.95 -> 6.41 ms a pass (idle lanes that end a round: 6 6.93, 12 6.41, 20 6.42).
-constexpr int kTrackRefill = 12;
+// It needs waves of more than kTrackRounds paths per resident lane: with fewer there is little or
+// nothing to refill a lane with, and the states cost registers (119) and steps.  128x128 pixels, depth
+// 4, us a pass, plain / queue: 32k paths 784 / 809, 64k 808 / 849, 128k 898 / 927, 256k 1121 / 1081,
+// 512k 1778 / 1648; depth 20: 1123 / 1169, 1329 / 1379, 1597 / 1681, 1965 / 1938, 2829 / 2750 (75,776
+// lanes resident).
+constexpr int kTrackRefill = 12, kTrackRounds = 2;
 template <bool SPH>
 __global__ void __launch_bounds__(256) k_track_queue(DevScene sc, PathState p, int bounce) {
   const int n = *ext_count(p, bounce);
@@ -3300,14 +3305,17 @@ void launch_shadow(const DevScene& s, const PathState& p, const Framebuffer& fb,
     });
   });
 }
-void launch_track(const DevScene& s, const PathState& p, int bounce, int grid, cudaStream_t st) {
+void launch_track(const DevScene& s, const PathState& p, int bounce, int paths, int grid, cudaStream_t st) {
   if (s.algo == TT_ALGO_PT2) return;  // the null-path tracer tracks inside its shade stage
   if (s.atmosphere && !s.wide) {
+    bool queue = false;
     with_bool(s.num_spheres > 0, [&](auto S) {
       auto* k = k_track_queue<decltype(S)::value>;
-      k<<<full_grid(k, blk(s)), blk(s), 0, st>>>(s, p, bounce);
+      const int b = blk(s), g = full_grid(k, b);
+      queue = paths > kTrackRounds * g * b;
+      if (queue) k<<<g, b, 0, st>>>(s, p, bounce);
     });
-    return;
+    if (queue) return;
   }
   with_bool(s.num_spheres > 0, [&](auto S) {
     with_bool(s.wide != 0, [&](auto W) {

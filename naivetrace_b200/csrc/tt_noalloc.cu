@@ -172,7 +172,7 @@ extern "C" tt_status tt_render_pass_noalloc(tt_ctx* ctx, int32_t spp, uint64_t s
     launch_shadow(scene, p, fb, b, false, nullptr, grid, st);
     launch_flush(scene, p, fb, b, grid, st);
     launch_extend(scene, p, b, false, nullptr, grid, st);
-    if (scene.num_media > 0) launch_track(scene, p, b, grid, st);
+    if (scene.num_media > 0) launch_track(scene, p, b, (int)paths, grid, st);
     launch_shade(scene, p, b, grid, st);
   }
   launch_shadow(scene, p, fb, depth, false, nullptr, grid, st);
