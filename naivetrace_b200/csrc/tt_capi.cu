@@ -1576,10 +1576,21 @@ static tt_status guide_train(tt_ctx* c, long long paths) {
 constexpr int kFewPaths = 1 << 14;
 constexpr int kFewUniformPaths = 1 << 16;
 static bool uniform_shading(const DevScene& s) { return s.num_media == 0 && s.sort_shading == 0; }
-static int whole_paths(const DevScene& s) {
+// Through an atmosphere a bounce of k_paths is long (its walks, and 380 bytes of spills per thread), so
+// with few bounces to go it takes fewer paths, or none.  Planet 128x128, us per pass, k_paths /
+// wavefront: whole waves of 16k paths 566 / 532 (depth 3), 689 / 722 (depth 4), of 4k 350 / 507 (depth
+// 3); from a bounce with two to go 777 / 744 (32k paths, depth 4), 1124 / 1093 (128k, depth 5), with
+// three to go 915 / 939 (32k, depth 5), 973 / 1127 (32k, depth 6).
+constexpr int kAtmosphereWhole = 4, kAtmosphereTail = 3;  // bounces
+static int whole_paths(const DevScene& s, int rounds) {
+  if (s.atmosphere && rounds < kAtmosphereWhole) return kFewPaths / 2;
   return uniform_shading(s) && !s.nodes4_bytes ? kFewUniformPaths : kFewPaths;
 }
 static int tail_paths(const DevScene& s) { return uniform_shading(s) ? kFewUniformPaths : kFewPaths; }
+// Whether k_paths may take over from bounce b on: after the guided bounces, from the second on.
+static bool tail_from(const DevScene& s, int b, int rounds) {
+  return b >= std::max(2, s.guide ? s.guide_depth : 0) && !(s.atmosphere && rounds - b < kAtmosphereTail);
+}
 
 // Starts a new wave's queue-length reports.
 static void next_wave_tag(tt_ctx* c) {
@@ -1663,21 +1674,20 @@ static tt_status render_range(tt_ctx* c, int32_t spp, uint64_t seed, int32_t pb,
     // bounces' few paths as whole paths again (after the guided bounces).  Not with guiding
     // records, nor when single launches are timed or counted.
     const bool whole = !c->dev.guide_record && !timing && c->dev.algo == TT_ALGO_PT && !c->dev.wide;
-    const bool fused = whole && !c->dev.guide && w.wave_paths <= whole_paths(c->dev) &&
+    const bool fused = whole && !c->dev.guide && w.wave_paths <= whole_paths(c->dev, rounds) &&
                        launch_paths(c->dev, c->ps, c->fb, w, -1, rounds, INT_MAX, kFlushNone, c->d_stats, c->stream);
     if (!fused) {
       if (whole) next_wave_tag(c);
       else c->ps.host_counts = nullptr;
       launch_generate(c->dev, c->ps, c->fb, w, grid, c->stream);
       launches++;
-      const int tail = std::max(2, c->dev.guide ? c->dev.guide_depth : 0);
       int b = 0;
       for (; b < rounds; ++b) {
         timed(1, [&] { launch_shadow(c->dev, c->ps, c->fb, b, counting, c->d_stats + 2, grid, c->stream); });
         ++shadow_launches;
         if (c->dev.guide_record) launch_flush(c->dev, c->ps, c->fb, b, grid, c->stream);
         // The launches of bounce b - 1 keep the device busy while the host reads its count.
-        if (c->ps.host_counts && b >= tail && reported_count(c, b - 1) <= (unsigned)tail_paths(c->dev) &&
+        if (c->ps.host_counts && tail_from(c->dev, b, rounds) && reported_count(c, b - 1) <= (unsigned)tail_paths(c->dev) &&
             launch_paths(c->dev, c->ps, c->fb, w, b, rounds, INT_MAX, kFlushNone, c->d_stats, c->stream)) {
           launches += 2;
           break;
@@ -2647,7 +2657,6 @@ static tt_status render_views(tt_ctx* c, const tt_view* views, int32_t n, uint64
   auto wave = [&](cudaStream_t s, bool eager) {
     int k = 2;
     const bool whole = !sc.guide_record && sc.algo == TT_ALGO_PT && !sc.wide;
-    const int tail = std::max(2, sc.guide ? sc.guide_depth : 0);
     if (eager && whole) next_wave_tag(c);
     else ps.host_counts = nullptr;
     cudaMemsetAsync(ps.counters, 0, kCountersPerBounce * (size_t)(rounds + 3) * sizeof(int), s);
@@ -2658,12 +2667,12 @@ static tt_status render_views(tt_ctx* c, const tt_view* views, int32_t n, uint64
       launch_flush(sc, ps, fb, b, grid, s);
       k += 2;
       if (eager) {
-        if (ps.host_counts && b >= tail && reported_count(c, b - 1) <= (unsigned)tail_paths(sc) &&
+        if (ps.host_counts && tail_from(sc, b, rounds) && reported_count(c, b - 1) <= (unsigned)tail_paths(sc) &&
             launch_paths(sc, ps, fb, none, b, rounds, INT_MAX, kFlushNow, c->d_stats, s)) {
           ++k;
           break;
         }
-      } else if (whole && b >= tail && b % 4 == 0 &&
+      } else if (whole && b % 4 == 0 && tail_from(sc, b, rounds) &&
                  launch_paths(sc, ps, fb, none, b, rounds, tail_paths(sc), kFlushCaptured, c->d_stats, s)) {
         k += 2;
       }
