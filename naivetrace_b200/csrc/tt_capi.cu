@@ -160,8 +160,10 @@ using HostArray = std::vector<T, NoInitAlloc<T>>;
 // one driver thread and pays the caller's page faults in it.  A million rays through a closest-hit
 // and an occlusion query: 12.6 -> 3.8 ms with it and device buffers from the pool; a 1920x1080
 // frame's host side 5.9 -> 1.5 ms (with the sample counts no longer kept per pixel).  Small copies
-// are left to the driver.  Returns when the caller's memory may be used again (to the host: holds
-// the data).
+// are left to the driver, and so is memory that is not pageable: page-locked memory is the DMA's own
+// source or target (a 1920x1080 frame into it 0.48 ms, through the blocks 1.18), and managed or device
+// memory is not the host's to touch here.  Returns when the caller's memory holds the data (to the
+// host) or may be used again (to the device; page-locked memory once the stream has come past the copy).
 struct HostCopy {
   void* host;
   void* dev;
@@ -169,18 +171,36 @@ struct HostCopy {
 };
 constexpr size_t kStageChunk = size_t(1) << 20;   // bytes per chunk (a host pool block)
 constexpr size_t kStageMin = size_t(2) << 20;     // below, the driver's own path is as fast
+static bool is_pageable(const void* p) {
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return a.type == cudaMemoryTypeUnregistered;
+}
 static cudaError_t staged_copy(int device, cudaStream_t stream, const HostCopy* copies, int count, bool to_device) {
+  // Bit k: copy k goes through the blocks.
+  unsigned staged = 0u;
   size_t total = 0;
-  for (int k = 0; k < count; ++k) total += copies[k].bytes;
-  if (total < kStageMin) {
-    cudaError_t e = cudaSuccess;
-    for (int k = 0; k < count && e == cudaSuccess; ++k) {
-      if (copies[k].bytes == 0) continue;
-      e = to_device ? cudaMemcpyAsync(copies[k].dev, copies[k].host, copies[k].bytes, cudaMemcpyHostToDevice, stream)
-                    : cudaMemcpyAsync(copies[k].host, copies[k].dev, copies[k].bytes, cudaMemcpyDeviceToHost, stream);
-    }
+  for (int k = 0; k < count; ++k) {
+    if (copies[k].bytes == 0 || !is_pageable(copies[k].host)) continue;
+    staged |= 1u << k;
+    total += copies[k].bytes;
+  }
+  if (total < kStageMin) staged = 0u;
+  cudaError_t plain = cudaSuccess;
+  for (int k = 0; k < count && plain == cudaSuccess; ++k) {
+    if (copies[k].bytes == 0 || (staged >> k & 1u)) continue;
+    plain = to_device
+                ? cudaMemcpyAsync(copies[k].dev, copies[k].host, copies[k].bytes, cudaMemcpyHostToDevice, stream)
+                : cudaMemcpyAsync(copies[k].host, copies[k].dev, copies[k].bytes, cudaMemcpyDeviceToHost, stream);
+  }
+  if (staged == 0u || plain != cudaSuccess) {
     // A pageable source is staged by the driver before the call returns; results need the wait.
-    return e == cudaSuccess && !to_device ? cudaStreamSynchronize(stream) : e;
+    if (to_device && plain == cudaSuccess) return cudaSuccess;
+    const cudaError_t e = cudaStreamSynchronize(stream);
+    return plain != cudaSuccess ? plain : e;
   }
   std::vector<HostCopy> chunks;
   try {
@@ -189,7 +209,7 @@ static cudaError_t staged_copy(int device, cudaStream_t stream, const HostCopy* 
     return cudaErrorMemoryAllocation;
   }
   for (int k = 0; k < count; ++k)
-    for (size_t o = 0; o < copies[k].bytes; o += kStageChunk)
+    for (size_t o = 0; (staged >> k & 1u) && o < copies[k].bytes; o += kStageChunk)
       chunks.push_back(HostCopy{static_cast<char*>(copies[k].host) + o, static_cast<char*>(copies[k].dev) + o,
                                 std::min(kStageChunk, copies[k].bytes - o)});
   const int workers = (int)std::min<size_t>(chunks.size(), std::min(8u, std::max(1u, std::thread::hardware_concurrency())));
@@ -1930,6 +1950,7 @@ tt_status tt_intersect_batch(tt_ctx* c, const float* rays, int32_t n, int32_t* p
     const HostCopy out[4] = {{prim, dp, prim ? n4 : 0}, {t, dt, t ? n4 : 0}, {u, du, u ? n4 : 0}, {v, dv, v ? n4 : 0}};
     e = staged_copy(c->device, c->stream, out, 4, false);
   }
+  if (e != cudaSuccess) cudaStreamSynchronize(c->stream);  // no copy of the caller's memory left in flight
   m.free_all();
   if (e != cudaSuccess) return fail(c, TT_ERR_CUDA, cudaGetErrorString(e));
   return TT_OK;
@@ -1954,6 +1975,7 @@ tt_status tt_occluded_batch(tt_ctx* c, const float* rays, int32_t n, uint8_t* oc
   }
   const HostCopy out{occ, docc, occ ? (size_t)n : 0};
   if (e == cudaSuccess) e = staged_copy(c->device, c->stream, &out, 1, false);
+  if (e != cudaSuccess) cudaStreamSynchronize(c->stream);
   m.free_all();
   if (e != cudaSuccess) return fail(c, TT_ERR_CUDA, cudaGetErrorString(e));
   return TT_OK;
