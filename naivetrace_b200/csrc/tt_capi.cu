@@ -157,20 +157,23 @@ using HostArray = std::vector<T, NoInitAlloc<T>>;
 // Copies between pageable caller memory and the device, ordered on `stream`, through page-locked
 // blocks of the host pool: several threads move chunks between the caller's memory and their own
 // block while the DMA of other chunks runs.  A plain copy from or to pageable memory goes through
-// one driver thread and pays the caller's page faults in it.  A million rays through a closest-hit
-// and an occlusion query: 12.6 -> 3.8 ms with it and device buffers from the pool; a 1920x1080
-// frame's host side 5.9 -> 1.5 ms (with the sample counts no longer kept per pixel).  Small copies
-// are left to the driver, and so is memory that is not pageable: page-locked memory is the DMA's own
-// source or target (a 1920x1080 frame into it 0.48 ms, through the blocks 1.18), and managed or device
-// memory is not the host's to touch here.  Returns when the caller's memory holds the data (to the
-// host) or may be used again (to the device; page-locked memory once the stream has come past the copy).
+// one driver thread.  Left to the driver are small copies and memory that is not pageable:
+// page-locked memory is the DMA's own source or target (a 1920x1080 image into it 0.48 ms, through
+// the blocks 1.18), and managed or device memory is not the host's to touch here.  Returns when the
+// caller's memory holds the data (to the host) or may be used again (to the device; page-locked
+// memory once the stream has come past the copy).
 struct HostCopy {
   void* host;
   void* dev;
   size_t bytes;
 };
 constexpr size_t kStageChunk = size_t(1) << 20;   // bytes per chunk (a host pool block)
-constexpr size_t kStageMin = size_t(2) << 20;     // below, the driver's own path is as fast
+// Bytes of a direction from which the blocks are used.  Rays to the device and their hits back, us a
+// call, blocks / driver: 2.1 MB of rays 330-390 / 285, 3.2 MB 440 / 395, 4.2 MB 420 / 473, 6.4 MB 590 /
+// 672, 9.6 MB 800 / 975, 32 MB 1,880 / 4,420 (a line at 4 MiB: 280, 390, 482, 655, 700, 1,770).  An image
+// alone gains little or nothing: 2.8 MB 230-400 / 210-240, 11 MB 600-900 / 610-750, 25 MB 1,090-1,390 /
+// 1,280-1,350.
+constexpr size_t kStageMin = size_t(2) << 20;
 static bool is_pageable(const void* p) {
   cudaPointerAttributes a;
   if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
