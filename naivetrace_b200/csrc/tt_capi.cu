@@ -1731,14 +1731,17 @@ static tt_status render_range(tt_ctx* c, int32_t spp, uint64_t seed, int32_t pb,
       if (b == rounds) {
         timed(1, [&] { launch_shadow(c->dev, c->ps, c->fb, rounds, counting, c->d_stats + 2, grid, c->stream); });
         ++shadow_launches;
+        ++launches;
       }
+    } else {
+      ++launches;
     }
     // Finished paths into the pass framebuffer: with guiding records, k_flush after every
     // bounce (it also commits the records); without, one gather at the end of the wave.
     if (c->dev.guide_record) launch_flush(c->dev, c->ps, c->fb, rounds, grid, c->stream);
     else launch_gather(c->ps, c->fb, w, fused, grid, c->stream);
     k_tally<<<1, 32, 0, c->stream>>>(c->ps.counters, rounds, c->d_stats);
-    launches += 3;
+    launches += 2;
     cudaEventRecord(wave_ev[wave_index & 1], c->stream);
   }
   launch_accumulate(c->fb, c->d_acc, c->d_light, 3 * c->npix, c->stream);
@@ -2677,11 +2680,14 @@ static tt_status render_views(tt_ctx* c, const tt_view* views, int32_t n, uint64
   PathState& ps = c->ps;
   // One wave's launches.  eager: the host watches the queue lengths and ends the wave with whole
   // paths; in a captured wave the same launch sits behind several bounces and takes over where its
-  // own limit is met.  Returns the kernels launched.
+  // own limit is met.  Not when launches are profiled.  Returns the launches.
+  struct Launches {
+    int all, extend, shadow;
+  };
   WaveArgs none{};
   auto wave = [&](cudaStream_t s, bool eager) {
-    int k = 2;
-    const bool whole = !sc.guide_record && sc.algo == TT_ALGO_PT && !sc.wide;
+    Launches k{2, 0, 0};
+    const bool whole = !sc.guide_record && !c->profiling && sc.algo == TT_ALGO_PT && !sc.wide;
     if (eager && whole) next_wave_tag(c);
     else ps.host_counts = nullptr;
     cudaMemsetAsync(ps.counters, 0, kCountersPerBounce * (size_t)(rounds + 3) * sizeof(int), s);
@@ -2690,31 +2696,35 @@ static tt_status render_views(tt_ctx* c, const tt_view* views, int32_t n, uint64
     for (; b < rounds; ++b) {
       launch_shadow(sc, ps, fb, b, false, nullptr, grid, s);
       launch_flush(sc, ps, fb, b, grid, s);
-      k += 2;
+      k.all += 2;
+      ++k.shadow;
       if (eager) {
         if (ps.host_counts && tail_from(sc, b, rounds) && reported_count(c, b - 1) <= (unsigned)tail_paths(sc) &&
             launch_paths(sc, ps, fb, none, b, rounds, INT_MAX, kFlushNow, c->d_stats, s)) {
-          ++k;
+          ++k.all;
           break;
         }
       } else if (whole && b % 4 == 0 && tail_from(sc, b, rounds) &&
                  launch_paths(sc, ps, fb, none, b, rounds, tail_paths(sc), kFlushCaptured, c->d_stats, s)) {
-        k += 2;
+        k.all += 2;
       }
       launch_extend(sc, ps, b, false, nullptr, grid, s);
       if (sc.num_media > 0) launch_track(sc, ps, b, hw[0].wave_paths, grid, s);
       launch_shade(sc, ps, b, grid, s);
       if (sc.guide && b < sc.guide_depth) launch_guide(sc, ps, b, s);
-      k += 1 + (sc.num_media > 0) + shade_launches(sc, ps, b) + (sc.guide && b < sc.guide_depth);
+      ++k.extend;
+      k.all += 1 + (sc.num_media > 0) + shade_launches(sc, ps, b) + (sc.guide && b < sc.guide_depth);
     }
     if (b == rounds) {
       launch_shadow(sc, ps, fb, rounds, false, nullptr, grid, s);
       launch_flush(sc, ps, fb, rounds, grid, s);
-      k += 2;
+      k.all += 2;
+      ++k.shadow;
     }
     k_tally<<<1, 32, 0, s>>>(ps.counters, rounds, c->d_stats);
     launch_wave_advance(d_idx, s);
-    return k + 1;
+    ++k.all;
+    return k;
   };
   cudaEventCreate(&ev0);
   cudaEventCreate(&ev1);
@@ -2723,14 +2733,15 @@ static tt_status render_views(tt_ctx* c, const tt_view* views, int32_t n, uint64
   int done_waves = 0;
   for (cudaEvent_t& e : wave_end)
     if ((st = check(cudaEventCreate(&e))) != TT_OK) return st;
-  uint64_t launches = (uint64_t)wave(c->stream, true);  // eager first wave
+  const Launches first = wave(c->stream, true);  // eager first wave
+  Launches later{0, 0, 0};                       // per replayed wave
   cudaEventRecord(wave_end[0], c->stream);
   ++done_waves;
   if ((st = check(cudaGetLastError())) != TT_OK) return st;
   if (nwaves > 1) {
     prepare_paths_launch(sc);
     if ((st = check(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal))) != TT_OK) return st;
-    const int per_wave = wave(c->stream, false);
+    later = wave(c->stream, false);
     cudaError_t ce = cudaStreamEndCapture(c->stream, &graph);
     if (ce == cudaSuccess) ce = cudaGraphInstantiate(&exec, graph, 0);
     if ((st = check(ce)) != TT_OK) return st;
@@ -2738,7 +2749,6 @@ static tt_status render_views(tt_ctx* c, const tt_view* views, int32_t n, uint64
       if (c->stop.load()) { stopped = true; break; }
       if ((st = check(cudaGraphLaunch(exec, c->stream))) != TT_OK) return st;
       cudaEventRecord(wave_end[done_waves], c->stream);
-      launches += (uint64_t)per_wave;
     }
   }
   launch_resolve_views(d_acc, d_light, d_views, n, (int)npix_total, d_rgb, c->stream);
@@ -2758,9 +2768,9 @@ static tt_status render_views(tt_ctx* c, const tt_view* views, int32_t n, uint64
     if (w < done_waves) cudaEventElapsedTime(&c->views_done_ms[v], ev0, wave_end[w]);
   }
   c->stats.pass_ms += ms;
-  c->stats.kernel_launches += launches + 1;
-  c->stats.extend_launches += (uint64_t)done_waves * rounds;
-  c->stats.shadow_launches += (uint64_t)done_waves * (rounds + 1);
+  c->stats.kernel_launches += (uint64_t)first.all + (uint64_t)(done_waves - 1) * later.all + 1;
+  c->stats.extend_launches += (uint64_t)first.extend + (uint64_t)(done_waves - 1) * later.extend;
+  c->stats.shadow_launches += (uint64_t)first.shadow + (uint64_t)(done_waves - 1) * later.shadow;
   c->stats.paths += (uint64_t)std::min<long long>(paths, (long long)done_waves * cap);
   cleanup();
   if (c->dev.guide_record && !stopped && c->gparams.train == 1) {

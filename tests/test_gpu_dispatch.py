@@ -24,3 +24,45 @@ def _bounces(scene, spp, depth, **kw):
 @pytest.mark.parametrize("side,spp,depth,bounces", [(128, 1, 3, 3), (64, 2, 3, 0), (128, 1, 4, 0), (128, 2, 4, 4)])
 def test_few_bounces_through_an_atmosphere(side, spp, depth, bounces):
     assert _bounces(scenes.planet_atmosphere(side, side), spp, depth) == bounces
+
+
+@pytest.mark.parametrize("side,spp,bounces", [(64, 1, 0), (320, 2, None)])
+def test_launch_counts_of_a_pass(side, spp, bounces):
+    """Cornell box (no media, one shader kind): every launch of the pass is counted once."""
+    depth = 12
+    plain = GpuContext(scenes.cornell_box(side, side), make_params(max_ray_depth=depth))
+    plain.render(spp, seed=3)
+    s = plain.stats()
+    own = s["extend_launches"]
+    if bounces is None:
+        assert 2 <= own < depth  # ended as whole paths
+        # generate; shadow, extend, shade per bounce; shadow, whole paths; gather, tally, accumulate.
+        assert s["kernel_launches"] == 1 + 3 * own + 2 + 3
+        assert s["shadow_launches"] == own + 1
+    else:
+        assert own == bounces and s["shadow_launches"] == 0
+        assert s["kernel_launches"] == 1 + 3  # whole paths; gather, tally, accumulate
+    profiled = GpuContext(scenes.cornell_box(side, side), make_params(max_ray_depth=depth))
+    profiled.set_profiling(1)
+    profiled.render(spp, seed=3)
+    s = profiled.stats()
+    assert (s["extend_launches"], s["shadow_launches"]) == (depth, depth + 1)
+    assert s["kernel_launches"] == 1 + 3 * depth + 1 + 3
+
+
+def test_launch_counts_of_view_batches():
+    """The first wave of a batch may end as whole paths, the later (captured) ones launch every bounce;
+    with profiling on all waves do.  The rays are the same."""
+    depth = 12
+    views = [(scenes.CameraSpec(pos=(0.5, 0.5, -1.4 - 0.1 * k), dir=(0, 0, 1), xres=150, yres=100), 5) for k in range(2)]
+    rays = []
+    for wave_paths, profiling, waves in ((0, 0, 1), (70_000, 0, 3), (70_000, 1, 3)):
+        g = GpuContext(scenes.cornell_box(16, 16), make_params(max_ray_depth=depth, wave_paths=wave_paths))
+        g.set_profiling(profiling)
+        g.render_views(views, seed=3)
+        s = g.stats()
+        first = s["extend_launches"] - (waves - 1) * depth
+        assert first == depth if profiling else 2 <= first < depth
+        assert s["shadow_launches"] == first + 1 + (waves - 1) * (depth + 1)
+        rays.append([s[k] for k in ("paths", "extension_rays", "shadow_rays")])
+    assert rays[0] == rays[1] == rays[2]
