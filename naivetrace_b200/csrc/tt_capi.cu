@@ -1643,6 +1643,13 @@ static tt_status render_range(tt_ctx* c, int32_t spp, uint64_t seed, int32_t pb,
   if (pb < 0 || pe > c->npix || pb >= pe) return fail(c, TT_ERR_INVALID, "bad pixel range");
   TT_CUDA(c, cudaSetDevice(c->device));
   const int npix_range = pe - pb;
+  if (c->spp_count.empty() && npix_range < c->npix) {
+    try {
+      c->spp_count.assign(c->npix, c->spp_all);
+    } catch (const std::bad_alloc&) {
+      return fail(c, TT_ERR_CUDA, "out of host memory for the pixels' sample counts");
+    }
+  }
   const long long total = (long long)spp * npix_range;
   const int wave_limit = c->params.wave_paths > 0 ? c->params.wave_paths : kDefaultWave;
   int cap = (int)std::min<long long>(total, wave_limit);
@@ -1777,7 +1784,6 @@ static tt_status render_range(tt_ctx* c, int32_t spp, uint64_t seed, int32_t pb,
   c->stats.paths += (uint64_t)std::min<long long>(total, (long long)wave_index * cap);
   // Bookkeeping as in SimplePixelByPixelRenderingAlgo: the sample count of the pass is
   // added whether or not the pass completed.
-  if (c->spp_count.empty() && npix_range < c->npix) c->spp_count.assign(c->npix, c->spp_all);
   if (c->spp_count.empty()) c->spp_all += (uint64_t)spp;
   else
     for (int px = pb; px < pe; ++px) c->spp_count[px] += (uint64_t)spp;
