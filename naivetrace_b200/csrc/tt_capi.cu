@@ -1590,12 +1590,18 @@ static tt_status guide_train(tt_ctx* c, long long paths) {
 // walk alike.  128x128 pixels, us per pass, k_paths from the camera / wavefront with tail:
 //   Cornell box    16k paths 122 / 173 (depth 4), 330 / 378 (20); 64k 156 / 205, 451 / 500
 //   furnished room 16k paths 117 / 141, 395 / 427;                64k 128 / 152, 489 / 514
-//   terrain        16k paths 281 / 314, 351 / 379;                32k 406 / 332, 521 / 423
+//   terrain 128^2 (8 spheres, one shader kind)
+//                  16k paths 281 / 314, 351 / 379;                32k 406 / 332, 521 / 423
 //   materials      16k paths 232 / 238, 667 / 666;                32k 309 / 261, 926 / 808
 //   medium         16k paths 256 / 256, 841 / 837;                32k 297 / 271, 1087 / 983
-// and at 128k paths it loses in the room too (741 / 695 at depth 20).  Tail limits of 16k / 64k
-// paths, depth 20, 64k paths in the wave: Cornell box 604 / 500, terrain 535 / 449, room 577 /
-// 514; materials 966 / 1207, medium 1158 / 1269, spheres 981 / 1069, media mix 1885 / 2093.
+// and at 128k paths it loses in the room too (741 / 695 at depth 20).  As the tail of a larger wave it
+// takes over late: with byte boxes the walks, a chain of node fetches however many rays there are,
+// set the time, so the larger limit serves there whether the shading is uniform or not.  Tail limits of
+// 16k / 64k paths, us per pass: depth 20, 64k paths in the wave: Cornell box 604 / 500, terrain 128^2
+// 535 / 449, room 577 / 514; materials 966 / 1207, medium 1158 / 1269, spheres 981 / 1069, media mix
+// 1885 / 2093; three shader kinds (sorted), 641x359 x 1, depths 4, 8, 16: terrain 1024^2 with 32
+// spheres 1127 / 1100, 1635 / 1561, 1818 / 1648, terrain 512^2 904 / 883, 1330 / 1324, 1450 / 1380,
+// terrain 256^2 753 / 747, 1130 / 1148, 1251 / 1229.
 constexpr int kFewPaths = 1 << 14;
 constexpr int kFewUniformPaths = 1 << 16;
 static bool uniform_shading(const DevScene& s) { return s.num_media == 0 && s.sort_shading == 0; }
@@ -1609,7 +1615,9 @@ static int whole_paths(const DevScene& s, int rounds) {
   if (s.atmosphere && rounds < kAtmosphereWhole) return kFewPaths / 2;
   return uniform_shading(s) && !s.nodes4_bytes ? kFewUniformPaths : kFewPaths;
 }
-static int tail_paths(const DevScene& s) { return uniform_shading(s) ? kFewUniformPaths : kFewPaths; }
+static int tail_paths(const DevScene& s) {
+  return s.num_media == 0 && (s.sort_shading == 0 || s.nodes4_bytes) ? kFewUniformPaths : kFewPaths;
+}
 // Whether k_paths may take over from bounce b on: after the guided bounces, from the second on.
 static bool tail_from(const DevScene& s, int b, int rounds) {
   return b >= std::max(2, s.guide ? s.guide_depth : 0) && !(s.atmosphere && rounds - b < kAtmosphereTail);

@@ -66,3 +66,23 @@ def test_launch_counts_of_view_batches():
         assert s["shadow_launches"] == first + 1 + (waves - 1) * (depth + 1)
         rays.append([s[k] for k in ("paths", "extension_rays", "shadow_rays")])
     assert rays[0] == rays[1] == rays[2]
+
+
+# Paths at which the last bounces of a wave are handed over: 65,536 in scenes without media that do not
+# sort their hits or have byte boxes (16,384 primitives on), else 16,384.
+@pytest.mark.parametrize("name,limit", [("terrain", 1 << 16), ("cornell", 1 << 16), ("materials", 1 << 14),
+                                        ("media", 1 << 14)])
+def test_limit_of_the_last_paths(name, limit):
+    depth = 14
+    scene = {"terrain": lambda x, y: scenes.terrain_spheres(x, y, terrain_n=128, sphere_level=2, num_spheres=32,
+                                                            env_w=64, env_h=32),
+             "cornell": scenes.cornell_box, "materials": scenes.cornell_box_materials,
+             "media": scenes.cornell_box_media_mix}[name](500, 300)
+    g = GpuContext(scene, make_params(max_ray_depth=depth))
+    assert (g.stats()["bvh_node_bytes"] == 64) == (name == "terrain")
+    g.render(1, seed=3)
+    lengths = [int(q) for q in g.queue_lengths(depth)[:, 0]]
+    # From the third bounce on, by the length of the bounce before.
+    first = next((b for b in range(2, depth) if lengths[b - 1] <= limit), depth)
+    assert g.stats()["extend_launches"] == first
+    assert lengths[0] > (1 << 16)
