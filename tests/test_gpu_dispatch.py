@@ -2,7 +2,7 @@
 launch counts in the stats (closest-hit launches count bounces that run as their own)."""
 import pytest
 
-from naivetrace_b200 import scenes
+from naivetrace_b200 import abi, scenes
 from naivetrace_b200.algo import GpuContext
 from naivetrace_b200.scene import make_params
 
@@ -17,6 +17,18 @@ def _bounces(scene, spp, depth, **kw):
     assert s["error_flags"] == 0
     assert s["shadow_launches"] in (s["extend_launches"], s["extend_launches"] + 1)
     return s["extend_launches"]
+
+
+# Waves of at most 16,384 paths run as whole paths from their camera samples, in scenes without media,
+# sorted shading or byte boxes of at most 65,536.
+@pytest.mark.parametrize("name,limit", [("cornell_box", 1 << 16), ("guiding_room", 1 << 16),
+                                        ("cornell_box_materials", 1 << 14), ("spheres_box", 1 << 14),
+                                        ("cornell_box_media_mix", 1 << 14), ("planet_atmosphere", 1 << 14)])
+def test_limit_of_whole_waves(name, limit):
+    spp = limit // (64 * 64)
+    assert _bounces(getattr(scenes, name)(64, 64), spp, 9) == 0
+    assert _bounces(getattr(scenes, name)(64, 64), spp + 1, 9) >= 2
+    assert _bounces(getattr(scenes, name)(64, 64), spp, 9, algo=abi.ALGO_PT2) == 9
 
 
 # Few bounces through an atmosphere are faster as their own launches than as whole paths: waves of
