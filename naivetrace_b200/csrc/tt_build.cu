@@ -474,8 +474,13 @@ __global__ void k_write_nodes(int first, int count, uint32_t n, const Aabb* node
 }
 
 // Scenes of at least this many primitives get byte boxes in their 4-wide nodes: below, the
-// nodes and primitives stay in the L1 whatever their format (closest and any hit measured
-// 2-6 % slower with byte boxes in rooms of 20-40 triangles; 8-10 % faster on the terrain).
+// nodes and primitives stay in the L1 whatever their format.  Float / byte boxes, us a pass:
+//   terrain 1920x1080 x 4   4,482 primitives 5,322 / 5,392, 10,498 5,765 / 5,796, 18,760 5,960 / 6,003,
+//                           34,818 6,116 / 6,125, 75,040 6,691 / 6,623, 171,010 7,186 / 7,024,
+//                           686,082 8,172 / 7,785
+//   bumpy mesh in the Cornell box, 1024x1024 x 4   1,956 9,874 / 9,953, 7,972 11,322 / 10,953,
+//                           16,234 11,919 / 11,301, 32,292 12,525 / 11,947, 130,084 13,869 / 12,694
+// (rooms of 20-40 triangles: closest and any hit 2-6 % slower with byte boxes).
 constexpr uint32_t kNode4BytesMin = 16384;
 
 // Writes a 4-wide node of m children with float boxes (layout in tt_build.h).
@@ -502,7 +507,10 @@ __device__ void write_node4_float(float4* d, const Aabb* box, const int* ref, in
 // 1/253 of the children's extent (at least 2^-22 of the coordinates, so that a step is never
 // lost in the float origin) and its origin one step below the lowest plane; lower planes round
 // down and upper planes up with a margin of 1/32 step for the traversal's rounding.  An empty
-// slot has an inverted box (never met) and the first child's reference.
+// slot has an inverted box and the first child's reference.  The box is met only by a ray so far away
+// that the widening of its exit distances exceeds 255 steps; the first child is then visited again.
+// It is a leaf: a node keeps an empty slot only if none of its children is an inner node (k_collapse4),
+// so the stack, counted with four entries above every node, holds that too.
 __device__ void write_node4_bytes(float4* d, const Aabb* box, const int* ref, int m) {
   float org[3], step[3];
   unsigned qlo[3], qhi[3];
@@ -554,7 +562,6 @@ __global__ void k_collapse4(const int4* frontier, int nfront, uint32_t n, const 
                             const int* right, const int* size, const int* offset, const unsigned char* emit,
                             const int* index, int* counter, int4* next, int* nnext, int* stack_need, int bytes,
                             float4* nodes4) {
-  constexpr int kEmpty = 0x7fffffff;
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nfront; t += gridDim.x * blockDim.x) {
     const int k = frontier[t].x, i4 = frontier[t].y;
     int slot[4] = {left[k], right[k], -1, -1};

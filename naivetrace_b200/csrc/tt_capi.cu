@@ -955,6 +955,7 @@ tt_status tt_upload_scene(tt_ctx* c) {
   s.wide = width_env && std::atoi(width_env) == 8;
   const bool binary_only = width_env && std::atoi(width_env) == 2;
   s.nodes4 = nullptr;
+  s.nodes4_bytes = 0;
   // The binary BVH is built on the device (PLOC) unless TT_BVH_BUILD=host asks for the
   // host binned-SAH builder.
   const char* build_env = std::getenv("TT_BVH_BUILD");

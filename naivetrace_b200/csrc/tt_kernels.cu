@@ -6,15 +6,21 @@
 //   generate  - wavelength selection, next-event estimation at the camera vertex
 //               (splatted to the pixel the light sample projects to), camera ray.
 //   extend    - closest hit of the queued extension rays (BVH traversal).
+//   track     - (media) the walk through the media in front of the hit, which may end the ray at a
+//               volume vertex.
+//   sort      - (scenes that mix shader kinds) orders the hits by shading key.
 //   shade     - MIS-weighted emission at the hit, Russian roulette, next-event estimation
 //               (emits a shadow ray), BSDF sampling (emits the next extension ray).
 //   shadow    - occlusion test; adds the NEE contribution of unoccluded rays.
 //   guide     - (guided scenes) the network on the vertices shade queued for guiding, then
 //               one-sample MIS of the BSDF and the learned mixture (emits the next ray).
-//   flush     - converts finished paths to RGB and adds them to the framebuffer; commits
-//               the path's training record when the guide is being trained.
-// Queues are appended with warp-aggregated atomics.  All kernels loop grid-stride over a
-// device-side count, so launch shapes are fixed (a multiple of the SM count).
+//   gather    - at the end of a wave: every pixel sums the RGB of its paths.
+//   flush     - in its place after every bounce of view batches and of passes that collect training
+//               records: finished paths into the framebuffer, their records committed.
+// Queues are appended with warp-aggregated atomics.  These kernels loop grid-stride over a
+// device-side count, or take it in chunks of 32 per warp with refilled lanes (closest_queue4,
+// any_queue4, k_track_queue), so launch shapes are fixed (a multiple of the SM count).  k_paths runs
+// all stages of few paths in one launch, bounce by bounce in registers, by the same functions.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -389,7 +395,7 @@ __device__ __forceinline__ void trace_ww(const BvhRef& bvh, TraceState& s, int* 
 //   bytes on it, rounded outwards.
 // In large scenes the traversal is bound by the L1 (per-lane node reads took 56-63 % of its data
 // pipe at a 48 % hit rate with float boxes) and by issue about equally; byte boxes halve the
-// former (31-37 %).  In small scenes every node hits the L1 and decoding only adds instructions.
+// former (31-36 %).  In small scenes every node hits the L1 and decoding only adds instructions.
 // A plane byte b becomes a float without a conversion: the byte placed in bits 8-15 of the
 // mantissa of 1.0 is 1 + b 2^-15, so t = a + b s / d = fma(1 + b 2^-15, 2^15 s / d, a - 2^15 s / d),
 // a = (p - o) / d, whose rounding (2^-9 of a grid step) the builder's outward margin of 1/32 step
@@ -559,10 +565,14 @@ __device__ __forceinline__ int visit_node4_any(const float4* __restrict__ nodes4
 // Byte boxes contain the float boxes, so a traversal of them meets every leaf that the float
 // boxes' traversal meets, and rarely one more: a float slab test can lose a box that the ray
 // touches within rounding of an edge (about one ray in 10^8 on the terrain), and then misses what
-// it holds.  So that hits do not depend on the node format, a hit in a tree of byte boxes counts
-// when the ray meets the leaf's box in the float test (it then meets every box around it, slab
-// distances being monotone in the planes): tested on the primitive's own box, which lies in the
-// leaf's, and only if that fails on the leaf's.
+// it holds.  So that what is hit and what is missed does not depend on the node format, a hit in a
+// tree of byte boxes counts when the ray meets the leaf's box in the float test (it then meets every
+// box around it, slab distances being monotone in the planes): tested on the primitive's own box,
+// which lies in the leaf's, and only if that fails on the leaf's.  Which of several primitives within
+// rounding of each other along the ray is the closest hit can still depend on the format, as on the
+// order of the walk: of rays through edges a few in a million, of those through vertices up to 10^-3
+// (binary against float 4-wide nodes: a fifth of that), of those through interiors, seen from within a
+// few scene extents, less than one in five million.
 // A closest hit is not held to the nearest hit so far there (the caller passes no limit): the
 // error of a box's entry is one of the ray origin's scale, so the entry of a nearer hit's box can
 // lie behind an earlier hit of the neighbouring leaf, which the walk with float boxes, testing both
@@ -723,8 +733,8 @@ struct WarpShare {
   __device__ __forceinline__ bool more() const { return index(taken) < n; }
 };
 
-// Closest hits of the rays 0 .. n-1 of `job` on the 4-wide layout.  job.load(k, ...) gives ray
-// k, job.store(k, r, slot, t, b1, b2) takes its result (slot -1: no hit).  All 32 lanes of
+// Closest hits of the rays 0 .. n-1 of `job` on the 4-wide layout with byte boxes.  job.load(k, ...)
+// gives ray k, job.store(k, r, slot, t, b1, b2) takes its result (slot -1: no hit).  All 32 lanes of
 // every warp of the grid take part.
 template <bool COUNT, bool SPH, class Job>
 __device__ __forceinline__ void closest_queue4(const DevScene& sc, const Job& job, int n, unsigned int* err,
@@ -735,7 +745,11 @@ __device__ __forceinline__ void closest_queue4(const DevScene& sc, const Job& jo
   RayPre r;
   float tnear = 0.f, best_t = 0.f, b1 = 0.f, b2 = 0.f;
   int best = -1, best_prim = 0, cur = kNoNode, leaf = kNoNode, sp = 0, ray = -1;
-  bool check = false;  // the ray's hits are tested against the leaf's float box
+  // Whether the ray's hits are tested against their leaf's float box as they are found.  Not in its
+  // first walk, whose result alone is tested; if that fails the ray walks again.  Testing every hit at
+  // once takes as long (terrain x 16 43.9 ms both ways, x 4 12.6) but decides about one in 10^7 rays
+  // through edges otherwise, so this form stays.
+  bool check = false;
   for (;;) {
     bool idle = cur == kNoNode && leaf == kNoNode;
     if (idle && ray >= 0) {
@@ -813,7 +827,7 @@ __device__ __forceinline__ void closest_queue4(const DevScene& sc, const Job& jo
   }
 }
 
-// Any hit of the rays 0 .. n-1 of `job` on the 4-wide layout.  job.store(k, r, slot).
+// Any hit of the rays 0 .. n-1 of `job` on the 4-wide layout with byte boxes.  job.store(k, r, slot).
 template <bool COUNT, bool SPH, class Job>
 __device__ __forceinline__ void any_queue4(const DevScene& sc, const Job& job, int n, unsigned int* err,
                                            TraceCounters* cnt) {
@@ -1588,9 +1602,8 @@ struct KeyHistogram {
   }
 };
 
-// Closest hit of the queued extension rays: on the 4-wide layout (the default) the queue is
-// traversed with refilled lanes, on the binary and the 8-wide layouts one ray per thread over a
-// grid-stride loop.
+// Closest hit of the queued extension rays: on the 4-wide layout with byte boxes (large scenes) the
+// queue is traversed with refilled lanes, on the others one ray per thread over a grid-stride loop.
 struct ExtendJob {
   const DevScene& sc;
   const PathState& p;
@@ -2673,13 +2686,20 @@ struct NoGuide {
 // are idle.  The wavefront launches three or more kernels per bounce, each as long as its
 // slowest ray's chain of dependent fetches however few rays it has (13-20 us in a box of 34
 // triangles, 100-180 us on the terrain); here that chain is paid once per path: a
-// 64x64 box at one sample takes 0.17 ms instead of 0.49 ms.  What bounds it is the issue of one
-// warp's instruction stream (6-7 cycles each at one warp per scheduler); when it serves how many
-// paths is in tt_capi.cu (whole_paths, tail_paths).
+// 64x64 box at one sample takes 0.17 ms instead of 0.49 ms.  What bounds it is the latency of a
+// warp's instruction stream (17-24 cycles from one instruction to the next, 16-23 % of the issue
+// slots used with 4,096 paths spread over 2,960 warps); when it serves how many paths is in tt_capi.cu
+// (whole_paths, tail_paths).
 // The stages are the wavefront kernels' functions in their order per path, so the results are the
 // same.  first < 0: the wave's camera samples, the finished paths' RGB left in accum for k_gather;
 // else the paths of bounce `first`'s extension queue (their shadow rays of that bounce traced
 // already), whose spectral sums go to accum or, flush, straight to the framebuffer.
+// Blocks of 64 or 256 threads and refills at 8 or 24 idle lanes measured the same within 4 %.  The
+// register cap (five blocks per SM, with media four) spills 208-270 bytes per thread, with media 380.
+// Without it 16,384 paths of depth 16 take 277 us instead of 299 in the Cornell box, 542 / 605 in the
+// materials box and 399 / 344 on a terrain of 42,498 triangles.  With media 637 / 940 (planet) and 622 /
+// 782 (medium box), but that code rounds some sums otherwise than the wavefront kernels, whose results
+// these are to equal bit for bit.
 constexpr int kPathBlock = 128;
 constexpr int kPathRefill = 16;
 template <bool MEDIA, bool SPH, int L>
