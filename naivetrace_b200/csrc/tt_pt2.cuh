@@ -80,8 +80,8 @@ __device__ __forceinline__ float3 exp_maj(float3 maj, float x) {
   return f3(expf(-x * maj.x), expf(-x * maj.y), expf(-x * maj.z));
 }
 
-// AccumulateContributions(w, f, p) (media_integrator.cxx:231-238) for two matrices with the same f: wa_ij *= f_j / f_i and
-// wb_ij *= p_j / f_i.
+// AccumulateContributions(w, f, p) (media_integrator.cxx:231-238) for two matrices with the same f:
+// wa_ij *= f_j / f_i and wb_ij *= p_j / f_i.
 __device__ __forceinline__ void m33_acc2(M33f& wa, M33f& wb, float3 f, float3 p) {
   const float inv[3] = {1.f / f.x, 1.f / f.y, 1.f / f.z}, fj[3] = {f.x, f.y, f.z}, pj[3] = {p.x, p.y, p.z};
 #pragma unroll
@@ -93,11 +93,27 @@ __device__ __forceinline__ void m33_acc2(M33f& wa, M33f& wb, float3 f, float3 p)
     }
 }
 
+// The same with p = f: both by f_j / f_i.
+__device__ __forceinline__ void m33_acc_same(M33f& wa, M33f& wb, float3 f) {
+  const float inv[3] = {1.f / f.x, 1.f / f.y, 1.f / f.z}, fj[3] = {f.x, f.y, f.z};
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      const float q = fix_nan(inv[i] * fj[j]);
+      wa.a[3 * i + j] = fix_nan(wa.a[3 * i + j] * q);
+      wb.a[3 * i + j] = fix_nan(wb.a[3 * i + j] * q);
+    }
+}
+
 // nullpath::Tracking on one segment: hero-wavelength delta tracking.  Returns true at a
 // real collision, at distance *t_out.  At most 10^4 steps (then no collision).
-// The three ends of a step choose factors and share one accumulation: k_shade2 was bound by
-// instruction fetch (11 of 18 cycles per issue), and with an accumulation per end and matrix this
-// loop alone held six copies of it (pt2 in mixed media 320x240 x 8: 10.3 -> 9.6 ms).
+// Collisions, null or real, choose factors and share one accumulation, and the segment's end has one
+// of half its products: k_shade2 was bound by instruction fetch (11 of 18 cycles per issue), and with
+// an accumulation per event and matrix this loop alone held six copies of it (pt2 in mixed media
+// 320x240 x 8: 10.3 -> 9.6 ms).  With the end sharing the collisions' accumulation as well, walks of
+// few collisions pay for products that cancel (planet 128x128 x 1, depth 12: 2,808 us instead of
+// 2,745, before either 2,748; mixed media x 16, depth 25: 5,065 instead of 5,095, before 5,240).
 template <class R>
 __device__ __forceinline__ bool track_segment2(const DevScene& sc, int medium, float3 org, float3 dir, float len,
                                                M33f& ft, M33f& fn, R& rng, Lambda l, float* t_out) {
@@ -108,25 +124,20 @@ __device__ __forceinline__ bool track_segment2(const DevScene& sc, int medium, f
     const float tlocal = fminf(kLargeNumber, -logf(1.f - rng.uniform()) * mfp);
     const float3 tr = exp_maj(maj, fminf(tlocal, len - t));
     t += tlocal;
-    float3 f = tr, pn = tr;
-    bool collided = false;
-    const bool end = t >= len;
-    if (!end) {
-      float3 ss, st;
-      coeffs2(sc, medium, org + dir * t, l, &ss, &st);
-      const float3 sn = maj - st;
-      const float prob_n = sn.x * mfp;
-      if (rng.uniform() < prob_n) {
-        f = mul(tr, sn);
-        pn = mul(tr, maj);
-      } else {
-        f = mul(tr, st);
-        collided = true;
-      }
+    if (t >= len) {
+      m33_acc_same(ft, fn, tr);
+      return false;
     }
+    float3 ss, st;
+    coeffs2(sc, medium, org + dir * t, l, &ss, &st);
+    const float3 sn = maj - st;
+    const bool collided = !(rng.uniform() < sn.x * mfp);
+    const float3 f = mul(tr, collided ? st : sn), pn = collided ? tr : mul(tr, maj);
     m33_acc2(ft, fn, f, pn);
-    if (collided) *t_out = t;
-    if (end || collided) return collided;
+    if (collided) {
+      *t_out = t;
+      return true;
+    }
   }
   return false;
 }
@@ -146,16 +157,13 @@ __device__ __forceinline__ void transmit_segment2(const DevScene& sc, int medium
     const float tlocal = fminf(kLargeNumber, -logf(1.f - rng.uniform()) * mfp);
     const float3 tr = exp_maj(maj, fminf(tlocal, len - t));
     t += tlocal;
-    float3 f = tr, pn = tr;
-    const bool end = t >= len;
-    if (!end) {
-      float3 ss, st;
-      coeffs2(sc, medium, org + dir * t, l, &ss, &st);
-      f = mul(tr, maj - st);
-      pn = mul(tr, maj);
+    if (t >= len) {
+      m33_acc_same(st_, sn_, tr);
+      break;
     }
-    m33_acc2(st_, sn_, f, pn);
-    if (end) break;
+    float3 ss, st;
+    coeffs2(sc, medium, org + dir * t, l, &ss, &st);
+    m33_acc2(st_, sn_, mul(tr, maj - st), mul(tr, maj));
     if (sn_.a[0] > kLargeNumber && sn_.a[4] > kLargeNumber && sn_.a[8] > kLargeNumber) {
 #pragma unroll
       for (int k = 0; k < 9; ++k) sn_.a[k] = INFINITY;
@@ -415,8 +423,12 @@ __global__ void __launch_bounds__(256) k_shade2(DevScene sc, PathState p, int bo
         }
         acc = acc + mis2<MEDIA>(sc, mul(rad, beta), has_last, last_pdf, last_delta, other, wt, wtn);
       }
+      // (Without media at the surface's own site: 128x128 x 16 in the materials box, depth 12, 1,639 us
+      // instead of 1,676 behind both; with media one call for both kinds of vertex.)
+      if (!MEDIA && sc.sample_lights)
+        nee2<MEDIA>(sc, p, bounce + 1, slot, rng, l, beta, wi, &s, rough, -1, vpos, mt, wt);
     }
-    if (!done && sc.sample_lights)
+    if (MEDIA && !done && sc.sample_lights)
       nee2<MEDIA>(sc, p, bounce + 1, slot, rng, l, beta, wi, volume ? nullptr : &s, rough, vmed, vpos, mt, wt);
     const int count = count0 + 1;
     if (!done && count > sc.max_path_nodes - 1) done = true;
