@@ -628,8 +628,12 @@ __device__ __forceinline__ bool test_leaf(const float4* __restrict__ tris, const
     bool hit;
     if (SPH && __float_as_int(cc.w) != 0) hit = intersect_sphere(r, a, b, tnear, best_t, &t);
     else hit = intersect_tri(r, xyz(a), xyz(b), xyz(cc), tnear, best_t, &t, &b1, &b2);
-    if (hit && (ANY || closer(t, __float_as_int(a.w), best_t, best_prim)) &&
-        (!BYTES || !check || leaf_box_met<SPH>(tris, r, start, count, a, b, cc, tnear, ANY ? best_t : INFINITY))) {
+    // (The leaf check as a condition of its own: joined to this one, where it folds to nothing without
+    // byte boxes, the compiled closest-hit loop of small scenes has 7 % more instructions.  Null-path
+    // tracer in the Cornell box, 128x128 x 1, depth 25: 1,198 us joined, 1,181 apart.)
+    if (hit && (ANY || closer(t, __float_as_int(a.w), best_t, best_prim))) {
+      if constexpr (BYTES)
+        if (check && !leaf_box_met<SPH>(tris, r, start, count, a, b, cc, tnear, ANY ? best_t : INFINITY)) continue;
       best = i;
       best_prim = __float_as_int(a.w);
       best_t = t;
