@@ -99,11 +99,17 @@ class HostPool {
     live_.erase(it);
     if (!b.pinned) {
       std::free(p);
-    } else if (kept_ + b.bytes <= kHostPoolKeep) {
-      free_.emplace(b.bytes, p);
-      kept_ += b.bytes;
     } else {
-      cudaFreeHost(p);
+      bool kept = false;
+      if (kept_ + b.bytes <= kHostPoolKeep) {
+        try {  // called from destructors and copy threads: nothing may leave here
+          free_.emplace(b.bytes, p);
+          kept_ += b.bytes;
+          kept = true;
+        } catch (const std::bad_alloc&) {
+        }
+      }
+      if (!kept) cudaFreeHost(p);
     }
   }
 
@@ -306,10 +312,9 @@ class CountAreas {
   static constexpr size_t kEntries = 1024;  // bounces: max_ray_depth <= 1000
   static unsigned long long* take() {
     {
-      std::lock_guard<std::mutex> g(mu());
-      if (!kept().empty()) {
-        unsigned long long* p = kept().back();
-        kept().pop_back();
+      std::lock_guard<std::mutex> g(mu_);
+      if (kept_ > 0) {
+        unsigned long long* p = areas_[--kept_];
         std::memset(p, 0, kEntries * sizeof(unsigned long long));  // no report of an earlier context's wave
         return p;
       }
@@ -326,9 +331,9 @@ class CountAreas {
   static void give(unsigned long long* p) {
     if (!p) return;
     {
-      std::lock_guard<std::mutex> g(mu());
-      if (kept().size() < 16) {
-        kept().push_back(p);
+      std::lock_guard<std::mutex> g(mu_);
+      if (kept_ < kKeep) {
+        areas_[kept_++] = p;
         return;
       }
     }
@@ -336,14 +341,10 @@ class CountAreas {
   }
 
  private:
-  static std::mutex& mu() {
-    static std::mutex* m = new std::mutex;
-    return *m;
-  }
-  static std::vector<unsigned long long*>& kept() {
-    static auto* v = new std::vector<unsigned long long*>;
-    return *v;
-  }
+  static constexpr int kKeep = 16;
+  inline static std::mutex mu_;
+  inline static unsigned long long* areas_[kKeep] = {};
+  inline static int kept_ = 0;
 };
 
 std::mutex g_pool_mutex;
